@@ -183,10 +183,10 @@ int sapb_batch_plan(sapb_batch *b, int n_clusters, const int *j_first, const int
     const float nr2 = (d->prec == SAPB_DOUBLE || d->order == SAPB_GRAPE5)
                           ? 0.0f : (float)(d->near_k * e2);
     cl[c] = BatchCluster{j_first[c], j_count[c], i_first, i_count[c], 1, 0,
-                         t_pred ? t_pred[c] : 0.0, e2, nr2, 0};
+                         t_pred ? t_pred[c] : 0.0, e2, nr2, 1};
     i_first += i_count[c];
     if (i_count[c] > 0) {
-      tpi[c] = tpi_rule(i_count[c], b->tpi_scale);
+      tpi[c] = cl[c].tpi = tpi_rule(i_count[c], b->tpi_scale);
       const int ti = 256 / tpi[c];
       tiles[c] = (i_count[c] + ti - 1) / ti;
       total_weight += (long long)tiles[c] * j_count[c];

@@ -3,6 +3,8 @@
 // sapb_batch.cu).  Work is described in device memory (BatchParams,
 // BatchCluster, BatchItem in sapb_internal.cuh), so the same graph runs any
 // step; per-cluster prediction times and softening are supported.
+#include <algorithm>
+
 #include "sapb_kernels.cuh"
 #include "sapb_launch.h"
 #include "sapb_pair.cuh"
@@ -257,76 +259,47 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
                      t[7 * kBT], t[8 * kBT], t[9 * kBT]};
       }
     }
-    // nearest neighbour: one rescan of the best tile (from L2)
-    unsigned long long key[2];
+    // combine rows in fixed order (the ring stages are idle: use the tiles
+    // area); the nearest neighbour's tile is its number within the slice
+    unsigned long long key[2], where[2];
+    __syncthreads();
+    double *red = reinterpret_cast<double *>(tiles);
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      key[p] = nn_key(kNoNgbDs2, -1);
-      if (best_tile[p] < 0) continue;
-      const int j0 = W.j_begin + best_tile[p] * kTJ;
-      const int cnt = min(kTJ, W.j_count - best_tile[p] * kTJ);
-      if (PREC == DOUBLE) {
-        const double4 *rec = reinterpret_cast<const double4 *>(pred + (size_t)j0 * C::REC);
-        for (int k = ty; k < cnt; k += tpi) {
-          double dx, dy, dz;
-          const double4 r0 = rec[k * C::RS + 0];
-          const double4 r1 = rec[k * C::RS + 1];
-          const float f2 = (float)pair_dr_dp(Id[p], r0, r1, dx, dy, dz);
-          if (f2 < kNoNgbDs2) key[p] = min(key[p], nn_key(f2, __double2loint(r1.w)));
-        }
-      } else {
-        const float4 *rec = reinterpret_cast<const float4 *>(pred + (size_t)j0 * C::REC);
-        for (int k = ty; k < cnt; k += tpi) {
-          float dx, dy, dz;
-          const float4 r0 = __ldg(rec + k * C::RS + 0);
-          const float4 r1 = __ldg(rec + k * C::RS + 1);
-          const float ds2 = pair_dr_mix(Im[p], r0, r1, dx, dy, dz);
-          if (ds2 < kNoNgbDs2) key[p] = min(key[p], nn_key(ds2, __float_as_int(r1.w)));
-        }
-      }
+      double *o = red + ((size_t)(ty * tit + tx) * 2 + p) * kResStride;
+      const NnSeen q = nn_seen(best[p], best_tile[p]);
+      o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
+      o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
+      o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
+      o[10] = __hiloint2double((int)q.d, (int)q.tile);
     }
-    // combine rows in fixed order (the ring stages are idle: use the tiles area)
     __syncthreads();
-    if (tpi > 1) {
-      double *red = reinterpret_cast<double *>(tiles);
-#pragma unroll
-      for (int p = 0; p < 2; p++) {
-        double *o = red + ((size_t)(ty * tit + tx) * 2 + p) * kResStride;
-        o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
-        o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
-        o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
-        o[10] = __longlong_as_double((long long)key[p]);
-      }
-      __syncthreads();
-      if (ty == 0) {
-#pragma unroll
-        for (int p = 0; p < 2; p++) {
-          for (int r = 1; r < tpi; r++) {
-            const double *o = red + ((size_t)(r * tit + tx) * 2 + p) * kResStride;
-            D[p].ax += o[0]; D[p].ay += o[1]; D[p].az += o[2]; D[p].pot += o[3];
-            D[p].jx += o[4]; D[p].jy += o[5]; D[p].jz += o[6];
-            D[p].sx += o[7]; D[p].sy += o[8]; D[p].sz += o[9];
-            key[p] = min(key[p], (unsigned long long)__double_as_longlong(o[10]));
-          }
-        }
-      }
-    }
     if (ty == 0) {
 #pragma unroll
       for (int p = 0; p < 2; p++) {
+        for (int r = 1; r < tpi; r++) {
+          const double *o = red + ((size_t)(r * tit + tx) * 2 + p) * kResStride;
+          D[p].ax += o[0]; D[p].ay += o[1]; D[p].az += o[2]; D[p].pot += o[3];
+          D[p].jx += o[4]; D[p].jy += o[5]; D[p].jz += o[6];
+          D[p].sx += o[7]; D[p].sy += o[8]; D[p].sz += o[9];
+        }
+        nn_rows<ORDER, PREC>(
+            tpi,
+            [&](int r) {
+              const double w = red[((size_t)(r * tit + tx) * 2 + p) * kResStride + 10];
+              return NnSeen{(unsigned)__double2hiint(w), (unsigned)__double2loint(w)};
+            },
+            [&](unsigned t) { return pred + (size_t)(W.j_begin + (int)t * kTJ) * C::REC; },
+            [&](unsigned t) { return min(kTJ, W.j_count - (int)t * kTJ); },
+            B.irec + (size_t)gi[p] * istr, key[p], where[p]);
         if (!valid[p]) continue;
         double *o = W.slot >= 0 ? B.part + (size_t)(W.slot + li[p]) * kResStride
                                 : B.res + (size_t)gi[p] * kResStride;
         o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
         o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
         o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
-        if (W.slot >= 0) {
-          o[10] = __longlong_as_double((long long)key[p]);
-          o[11] = 0.0;
-        } else {
-          o[10] = (double)__uint_as_float((unsigned int)(key[p] >> 32));
-          o[11] = (double)(int)(unsigned int)(key[p] & 0xffffffffu);
-        }
+        o[10] = __longlong_as_double((long long)key[p]);
+        o[11] = __longlong_as_double((long long)where[p]);
       }
     }
   }
@@ -336,31 +309,33 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
   }
 }
 
-// Sums the j-slices of clusters that were split (fixed slice order).
+// Sums the j-slices of every i and looks up its nearest neighbour's id: one
+// warp per i (reduce_one), a fixed grid striding over the active i.
+template <int ORDER, int PREC>
 __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs B) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int REC = PREC == DOUBLE ? 32 * pred_fields64(ORDER) : 16 * pred_fields(ORDER);
   const BatchParams &P = *B.par;
-  if (i >= P.total_i) return;
-  const int c = find_cluster(B.cl, P.n_clusters, i, [](const BatchCluster &q) { return q.i_first; });
-  if (c < 0) return;
-  const BatchCluster &CL = B.cl[c];
-  if (i >= CL.i_first + CL.i_count || CL.nslices <= 1) return;
-  const int li = i - CL.i_first;
-  double acc[10];
-#pragma unroll
-  for (int f = 0; f < 10; f++) acc[f] = 0.0;
-  unsigned long long key = nn_key(kNoNgbDs2, -1);
-  for (int s = 0; s < CL.nslices; s++) {
-    const double *o = B.part + ((size_t)CL.part_base + (size_t)s * CL.i_count + li) * kResStride;
-#pragma unroll
-    for (int f = 0; f < 10; f++) acc[f] += o[f];
-    key = min(key, (unsigned long long)__double_as_longlong(o[10]));
+  const int lane = threadIdx.x & 31;
+  const unsigned char *pred = reinterpret_cast<const unsigned char *>(B.pred);
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < P.total_i;
+       i += (gridDim.x * blockDim.x) >> 5) {
+    const int c =
+        find_cluster(B.cl, P.n_clusters, i, [](const BatchCluster &q) { return q.i_first; });
+    if (c < 0) continue;
+    const BatchCluster &CL = B.cl[c];
+    if (i >= CL.i_first + CL.i_count) continue;
+    const int S = CL.nslices;
+    const int sl = (CL.j_count + S - 1) / S;  // j per slice
+    double *out = B.res + (size_t)i * kResStride;
+    reduce_one<ORDER, PREC>(
+        S > 1 ? B.part + ((size_t)CL.part_base + (i - CL.i_first)) * kResStride : out,
+        (size_t)CL.i_count * kResStride, S, CL.tpi, lane, B.irec + (size_t)i * i_stride(ORDER),
+        out,
+        [&](int s, unsigned t) { return pred + (size_t)(CL.j_first + s * sl + (int)t * kTJ) * REC; },
+        [&](int s, unsigned t) {
+          return min(kTJ, min(sl, CL.j_count - s * sl) - (int)t * kTJ);
+        });
   }
-  double *w = B.res + (size_t)i * kResStride;
-#pragma unroll
-  for (int f = 0; f < 10; f++) w[f] = acc[f];
-  w[10] = (double)__uint_as_float((unsigned int)(key >> 32));
-  w[11] = (double)(int)(unsigned int)(key & 0xffffffffu);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -378,7 +353,8 @@ static cudaError_t launch_batch_t(const BatchArgs &B, int j_grid, int force_bloc
   if (B.do_predict && j_grid > 0)
     batch_predict_kernel<ORDER, PREC><<<(j_grid + 255) / 256, 256, 0, st>>>(B);
   batch_force_kernel<ORDER, PREC><<<force_blocks, kBT, C::SMEM, st>>>(B);
-  if (i_grid > 0) batch_reduce_kernel<<<(i_grid + 255) / 256, 256, 0, st>>>(B);
+  if (i_grid > 0)
+    batch_reduce_kernel<ORDER, PREC><<<std::min((i_grid + 7) / 8, 4 * force_blocks), 256, 0, st>>>(B);
   return cudaGetLastError();
 }
 

@@ -632,16 +632,12 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
     int rc = ensure_part(d, (size_t)P.ns * ni * kResStride);
     if (rc) return rc;
     A.out = d->part_d;
-    A.write_partials = 1;
   } else {
     A.out = res_dev;
-    A.write_partials = 0;
   }
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
-  if (P.ns > 1) {
-    ReduceArgs R{d->part_d, P.ns, ni, res_dev, cnt_dev};
-    CK(d, launch_reduce(R, d->stream));
-  }
+  const ReduceArgs R{A.out, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, A.iperm};
+  CK(d, launch_reduce(d->order, d->prec, R, d->stream));
   return SAPB_OK;
 }
 
@@ -770,10 +766,9 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
   A.ngb_list = ngb_list_dev;
   A.status = d->status_d;
   A.out = scratch;  // every (slice, valid i) record is written before it is read
-  A.write_partials = 1;
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
-  ReduceArgs R{scratch, P.ns, ni, res_dev, ngb_count_dev};
-  CK(d, launch_reduce(R, d->stream));
+  const ReduceArgs R{scratch, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, nullptr};
+  CK(d, launch_reduce(d->order, d->prec, R, d->stream));
   return SAPB_OK;
 }
 

@@ -14,7 +14,8 @@
 //   results, one record of 12 doubles per i:
 //     {acc0 acc1 acc2 pot jrk0 jrk1 jrk2 snp0 snp1 snp2 ds2min nnb|count}
 //   partial sums (scratch, used when the j range is split over S slices):
-//     12 doubles per (slice, i), same layout, NN stored as a 64-bit key.
+//     12 doubles per (slice, i), same layout, NN as a 64-bit key and where to
+//     look its id up.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -66,8 +67,7 @@ struct ForceArgs {
   double eps2;
   int nslices;        // S: j slices across blocks (slice s: tiles s, s+S, ...)
   int i_tiles;        // number of i tiles
-  double *out;        // results (S == 1) or partials (S > 1)
-  int write_partials; // 1: write 12-double partial records per (slice, i)
+  double *out;        // one 12-double record per (slice, i), see ReduceArgs
   int do_list;        // build neighbour lists
   int *ngb_count;     // [ni] (zeroed before launch)
   int *ngb_list;      // [ni * 256]
@@ -97,7 +97,7 @@ struct BatchCluster {
   int part_base;         // first partial record of this cluster
   double t_pred, eps2;
   float near_r2;         // mixed precision: near pairs (ds2 < near_r2) summed in FP64; 0 off
-  int pad_;
+  int tpi;               // threads per i of this cluster's items
 };
 struct BatchItem {
   int cluster;
@@ -126,12 +126,18 @@ struct BatchArgs {
   int *status;
 };
 
+// Records of the force kernel, one per (slice, i): the ten sums, then the
+// nearest neighbour as two 64-bit words (nn_rows in sapb_pair.cuh).
 struct ReduceArgs {
-  const double *part;
+  const double *part;  // == out when there is one slice
   int nslices;
   int ni;
   double *out;
-  const int *ngb_count;
+  // what the force call read: the nearest neighbour's id is looked up there
+  const void *pred;
+  int nj, tpi;
+  const double *irec;
+  const int *iperm;
 };
 
 }  // namespace sapb

@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // loop only keeps the tile's minimum ds2.  Neighbour list: when that minimum
 // is below h2, the warp rescans the tile cooperatively (lanes split the j)
 // and appends the hits.  Nearest neighbour: each thread remembers the tile
-// where its smallest ds2 first appeared and rescans only that tile, from L2,
-// after the loop.  Rescans recompute ds2 bit-identically (same rounded
+// where its smallest ds2 first appeared, and the reduction looks up the id
+// there (reduce_one).  Rescans recompute ds2 bit-identically (same rounded
 // operations).
 // ========================================================================
 // Unroll depth of the packed j loop (B200, 6th order, N = 2^20: 1 -> 501,
@@ -492,46 +492,21 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
     }
   }
 
-  // ---- nearest neighbour: one rescan of the best tile (from L2) ----
-  unsigned long long key[IP];
-#pragma unroll
-  for (int p = 0; p < IP; p++) {
-    key[p] = nn_key(kNoNgbDs2, -1);
-    if (best_tile[p] < 0) continue;
-    const int tile = slice + best_tile[p] * S;
-    const int cnt = min(kTJ, A.nj - tile * kTJ);
-    if (PREC == DOUBLE) {
-      const double4 *rec = reinterpret_cast<const double4 *>(pred + (size_t)tile * kTJ * C::REC);
-      for (int k = ty; k < cnt; k += TPI) {
-        double dx, dy, dz;
-        const double4 r0 = rec[k * C::RS + 0];
-        const double4 r1 = rec[k * C::RS + 1];
-        const float f2 = (float)pair_dr_dp(Id[p], r0, r1, dx, dy, dz);
-        if (f2 < kNoNgbDs2) key[p] = min(key[p], nn_key(f2, __double2loint(r1.w)));
-      }
-    } else {
-      const float4 *rec = reinterpret_cast<const float4 *>(pred + (size_t)tile * kTJ * C::REC);
-      for (int k = ty; k < cnt; k += TPI) {
-        float dx, dy, dz;
-        const float4 r0 = __ldg(rec + k * C::RS + 0);
-        const float4 r1 = __ldg(rec + k * C::RS + 1);
-        const float ds2 = pair_dr_mix(Im[p], r0, r1, dx, dy, dz);
-        if (ds2 < kNoNgbDs2) key[p] = min(key[p], nn_key(ds2, __float_as_int(r1.w)));
-      }
-    }
-  }
-
   // ---- combine rows (threads-per-i > 1), fixed order ----
+  unsigned long long key[IP], where[IP];  // nearest neighbour: see nn_rows
+  auto tile_rec = [&](unsigned t) { return pred + (size_t)t * kTJ * C::REC; };
+  auto tile_cnt = [&](unsigned t) { return min(kTJ, A.nj - (int)t * kTJ); };
   if (TPI > 1) {
     named_barrier(1, kBT);  // all consumer warps are past their last tile
     double *red = reinterpret_cast<double *>(tiles);
 #pragma unroll
     for (int p = 0; p < IP; p++) {
       double *o = red + ((size_t)(ty * C::TIT + tx) * IP + p) * kResStride;
+      const NnSeen q = nn_seen(best[p], best_tile[p] < 0 ? -1 : slice + best_tile[p] * S);
       o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
       o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
       o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
-      o[10] = __longlong_as_double((long long)key[p]);
+      o[10] = __hiloint2double((int)q.d, (int)q.tile);
     }
     named_barrier(1, kBT);
     if (ty != 0) return;
@@ -542,27 +517,34 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
         D[p].ax += o[0]; D[p].ay += o[1]; D[p].az += o[2]; D[p].pot += o[3];
         D[p].jx += o[4]; D[p].jy += o[5]; D[p].jz += o[6];
         D[p].sx += o[7]; D[p].sy += o[8]; D[p].sz += o[9];
-        key[p] = min(key[p], (unsigned long long)__double_as_longlong(o[10]));
       }
+      nn_rows<ORDER, PREC>(
+          TPI,
+          [&](int r) {
+            const double w = red[((size_t)(r * C::TIT + tx) * IP + p) * kResStride + 10];
+            return NnSeen{(unsigned)__double2hiint(w), (unsigned)__double2loint(w)};
+          },
+          tile_rec, tile_cnt, A.irec + (size_t)(valid[p] ? oi[p] : 0) * istr, key[p], where[p]);
     }
+  } else {
+#pragma unroll
+    for (int p = 0; p < IP; p++)
+      nn_rows<ORDER, PREC>(
+          1,
+          [&](int) { return nn_seen(best[p], best_tile[p] < 0 ? -1 : slice + best_tile[p] * S); },
+          tile_rec, tile_cnt, A.irec, key[p], where[p]);
   }
 
   // ---- write this block's results ----
 #pragma unroll
   for (int p = 0; p < IP; p++) {
     if (!valid[p]) continue;
-    double *o = A.write_partials ? A.out + ((size_t)slice * A.ni + oi[p]) * kResStride
-                                 : A.out + (size_t)oi[p] * kResStride;
+    double *o = A.out + ((size_t)slice * A.ni + oi[p]) * kResStride;
     o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
     o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
     o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
-    if (A.write_partials) {
-      o[10] = __longlong_as_double((long long)key[p]);
-      o[11] = 0.0;
-    } else {
-      o[10] = (double)__uint_as_float((unsigned int)(key[p] >> 32));
-      o[11] = (double)(int)(unsigned int)(key[p] & 0xffffffffu);
-    }
+    o[10] = __longlong_as_double((long long)key[p]);
+    o[11] = __longlong_as_double((long long)where[p]);
   }
 }
 
@@ -587,26 +569,22 @@ cudaError_t launch_wait_selftest(uint64_t limit_ns, int *status, cudaStream_t st
 }
 
 // ========================================================================
-// Cross-slice reduction: fixed slice order, so results are bit-stable.
+// Reduction over the slices, and the nearest neighbour's id: one warp per i
+// (reduce_one).  With one slice `part` is `out`.
 // ========================================================================
+template <int ORDER, int PREC>
 __global__ void __launch_bounds__(256) reduce_kernel(ReduceArgs R) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= R.ni) return;
-  double acc[10];
-#pragma unroll
-  for (int f = 0; f < 10; f++) acc[f] = 0.0;
-  unsigned long long key = nn_key(kNoNgbDs2, -1);
-  for (int s = 0; s < R.nslices; s++) {
-    const double *o = R.part + ((size_t)s * R.ni + i) * kResStride;
-#pragma unroll
-    for (int f = 0; f < 10; f++) acc[f] += o[f];
-    key = min(key, (unsigned long long)__double_as_longlong(o[10]));
-  }
-  double *w = R.out + (size_t)i * kResStride;
-#pragma unroll
-  for (int f = 0; f < 10; f++) w[f] = acc[f];
-  w[10] = (double)__uint_as_float((unsigned int)(key >> 32));
-  w[11] = (double)(int)(unsigned int)(key & 0xffffffffu);
+  constexpr int REC = PREC == DOUBLE ? 32 * pred_fields64(ORDER) : 16 * pred_fields(ORDER);
+  const int g = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (g >= R.ni) return;
+  const int i = R.iperm ? __ldg(R.iperm + g) : g;  // spatial mode: neighbours scan the same tiles
+  const unsigned char *pred = reinterpret_cast<const unsigned char *>(R.pred);
+  reduce_one<ORDER, PREC>(
+      R.part + (size_t)i * kResStride, (size_t)R.ni * kResStride, R.nslices, R.tpi, lane,
+      R.irec + (size_t)i * i_stride(ORDER), R.out + (size_t)i * kResStride,
+      [&](int, unsigned t) { return pred + (size_t)t * kTJ * REC; },
+      [&](int, unsigned t) { return min(kTJ, R.nj - (int)t * kTJ); });
 }
 
 // ========================================================================
@@ -767,10 +745,21 @@ cudaError_t launch_readj(int order, int first, int n, double ti, int predict, co
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(const ReduceArgs &R, cudaStream_t st) {
+template <int ORDER, int PREC>
+static cudaError_t launch_reduce_t(const ReduceArgs &R, cudaStream_t st) {
   if (R.ni <= 0) return cudaSuccess;
-  reduce_kernel<<<(R.ni + 255) / 256, 256, 0, st>>>(R);
+  reduce_kernel<ORDER, PREC><<<(R.ni + 7) / 8, 256, 0, st>>>(R);
   return cudaGetLastError();
+}
+
+cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, cudaStream_t st) {
+  if (order == GRAPE5 && prec == DOUBLESINGLE) return launch_reduce_t<GRAPE5, DOUBLESINGLE>(R, st);
+  if (order == GRAPE5) order = FOURTH;  // as the force kernels
+  if (order == FOURTH && prec == DOUBLESINGLE) return launch_reduce_t<FOURTH, DOUBLESINGLE>(R, st);
+  if (order == FOURTH && prec == DOUBLE) return launch_reduce_t<FOURTH, DOUBLE>(R, st);
+  if (order == SIXTH && prec == DOUBLESINGLE) return launch_reduce_t<SIXTH, DOUBLESINGLE>(R, st);
+  if (order == SIXTH && prec == DOUBLE) return launch_reduce_t<SIXTH, DOUBLE>(R, st);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace sapb

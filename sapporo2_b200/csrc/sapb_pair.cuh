@@ -524,4 +524,175 @@ __device__ __forceinline__ void list_rescan_dp(const IDp &I, bool want, int gi, 
 }
 
 
+// ---------------- nearest neighbour ----------------
+// The pair loops keep, per thread and i, only the smallest ds2 and the tile
+// it first appeared in.  Which record that was is looked up once per i, in
+// the reduction over the slices (nn_scan, one warp per i), and not at the end
+// of every slice, where each thread walked its own tile from L2, one record
+// after another (B200, a pass with and without: 192 clusters in a batch
+// 2.45 / 2.72 ms, 12983 i on 131072 j 3.96 / 4.06 ms, 600 i on 30011 j 114 /
+// 119 us of device time).
+// A block leaves two words per i: nn_key(ds2, id), and where to look:
+// kNnDone (the id is already there, or there is no neighbour) or the tile
+// (upper half) and the rows of it that saw this ds2 (lower half).
+constexpr unsigned long long kNnDone = ~0ull;
+
+struct NnSeen {
+  unsigned d;     // ds2, float bits
+  unsigned tile;  // ~0: none
+};
+__device__ __forceinline__ NnSeen nn_seen(float best, int tile) {
+  NnSeen s{__float_as_uint(kNoNgbDs2), ~0u};
+  if (tile >= 0) s = NnSeen{__float_as_uint(best), (unsigned)tile};
+  return s;
+}
+
+// Smallest nn_key over the records of rows `rows` (of tpi, a power of two)
+// of the `cnt` records at `tile_rec`; lane `lane` of `lanes` takes every
+// lanes-th record of a row.  ds2 is recomputed with the pair loop's rounded
+// operations.  `irec`: the i's record.
+template <int ORDER, int PREC>
+__device__ __forceinline__ unsigned long long nn_scan(const unsigned char *tile_rec, int cnt,
+                                                      unsigned rows, int tpi, int lane, int lanes,
+                                                      const double *irec) {
+  constexpr int RS = PREC == DOUBLE ? pred_fields64(ORDER) : pred_fields(ORDER);
+  unsigned long long key = nn_key(kNoNgbDs2, -1);
+  const double x = irec[0], y = irec[1], z = irec[2];
+  const int id = __double2loint(irec[7]);
+  while (rows) {
+    const int row = __ffs(rows) - 1;
+    rows &= rows - 1;
+    if (PREC == DOUBLE) {
+      const double4 *rec = reinterpret_cast<const double4 *>(tile_rec);
+      IDp I{};
+      I.x = x; I.y = y; I.z = z; I.id = id;
+#pragma unroll 2
+      for (int k = row + lane * tpi; k < cnt; k += lanes * tpi) {
+        double dx, dy, dz;
+        const double4 r0 = rec[(size_t)k * RS + 0];
+        const double4 r1 = rec[(size_t)k * RS + 1];
+        const float f2 = (float)pair_dr_dp(I, r0, r1, dx, dy, dz);
+        if (f2 < kNoNgbDs2) key = min(key, nn_key(f2, __double2loint(r1.w)));
+      }
+    } else {
+      const float4 *rec = reinterpret_cast<const float4 *>(tile_rec);
+      IMix I{};
+      I.xh = (float)x; I.yh = (float)y; I.zh = (float)z;
+      I.xl = (float)(x - (double)I.xh);
+      I.yl = (float)(y - (double)I.yh);
+      I.zl = (float)(z - (double)I.zh);
+      I.id = id;
+#pragma unroll 4
+      for (int k = row + lane * tpi; k < cnt; k += lanes * tpi) {
+        float dx, dy, dz;
+        const float4 r0 = __ldg(rec + (size_t)k * RS + 0);
+        const float4 r1 = __ldg(rec + (size_t)k * RS + 1);
+        const float ds2 = pair_dr_mix(I, r0, r1, dx, dy, dz);
+        if (ds2 < kNoNgbDs2) key = min(key, nn_key(ds2, __float_as_int(r1.w)));
+      }
+    }
+  }
+  return key;
+}
+
+// Combines the rows of a block for one i: the smallest ds2 and the rows of
+// its tile that saw it.  `row(r)` is row r's NnSeen, `rec(t)` the records of
+// tile t and `count(t)` their number.  When rows saw the same ds2 in
+// different tiles (an exact tie) the two words cannot name both, and the id
+// is looked up here.
+template <int ORDER, int PREC, typename Row, typename Rec, typename Count>
+__device__ __forceinline__ void nn_rows(int tpi, Row row, Rec rec, Count count,
+                                        const double *irec, unsigned long long &key,
+                                        unsigned long long &where) {
+  NnSeen m = row(0);
+  unsigned rows = 1u;
+  bool tie = false;
+  for (int r = 1; r < tpi; r++) {
+    const NnSeen q = row(r);
+    if (q.d < m.d) {
+      m = q;
+      rows = 1u << r;
+      tie = false;
+    } else if (q.d == m.d) {
+      if (q.tile == m.tile) rows |= 1u << r;
+      else tie = true;
+    }
+  }
+  key = nn_key(__uint_as_float(m.d), -1);
+  where = m.tile == ~0u ? kNnDone : ((unsigned long long)m.tile << 32) | rows;
+  if (tie && m.tile != ~0u) {
+    key = nn_key(kNoNgbDs2, -1);
+#pragma unroll 1
+    for (int r = 0; r < tpi; r++) {
+      const NnSeen q = row(r);
+      if (q.d == m.d && q.tile != ~0u)
+        key = min(key, nn_scan<ORDER, PREC>(rec(q.tile), count(q.tile), 1u << r, tpi, 0, 1, irec));
+    }
+    where = kNnDone;
+  }
+}
+
+// One i's records, one per slice, `step` doubles apart, summed by one warp:
+// lanes 0..9 and 16..25 sum one field each over the even and the odd slices
+// (fixed order, so results are bit-stable); one lane per slice finds the
+// smallest ds2, and the whole warp scans the tile it was seen in, eight
+// records per lane, for the id.  Small calls are bound by latency (one thread
+// per i used to walk slices x 12 words in a row; 48 i on 16384 j, 16 slices,
+// predictor and force included: 37.0 -> 32.2 us on B200), large ones by L2.
+// `part` may be `out`: the warp has read its records before it writes.
+// `rec(s, t)` / `count(s, t)`: records of tile t as slice s numbers them.
+template <int ORDER, int PREC, typename Rec, typename Count>
+__device__ __forceinline__ void reduce_one(const double *part, size_t step, int nslices, int tpi,
+                                           int lane, const double *irec, double *out, Rec rec,
+                                           Count count) {
+  const int f = lane & 15;
+  double acc = 0.0;
+  if (f < 10) {
+#pragma unroll 4
+    for (int s = lane >> 4; s < nslices; s += 2) acc += part[s * step + f];
+  }
+  acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+
+  const unsigned none = __float_as_uint(kNoNgbDs2);
+  unsigned d = none;
+  if (ORDER != GRAPE5)
+    for (int s = lane; s < nslices; s += 32)
+      d = min(d, (unsigned)__double2hiint(part[s * step + 10]));
+  d = __reduce_min_sync(0xffffffffu, d);
+  unsigned long long key = nn_key(kNoNgbDs2, -1);
+  if (d != none) {
+    for (int s0 = 0; s0 < nslices; s0 += 32) {
+      unsigned long long where = kNnDone;
+      bool todo = false;
+      if (s0 + lane < nslices) {
+        const double *o = part + (s0 + lane) * step;
+        const unsigned long long k = (unsigned long long)__double_as_longlong(o[10]);
+        where = (unsigned long long)__double_as_longlong(o[11]);
+        if ((unsigned)(k >> 32) == d) {
+          todo = where != kNnDone;
+          if (!todo) key = min(key, k);
+        }
+      }
+      unsigned m = __ballot_sync(0xffffffffu, todo);
+      while (m) {
+        const int src = __ffs(m) - 1;
+        m &= m - 1;
+        const unsigned long long w = __shfl_sync(0xffffffffu, where, src);
+        const unsigned t = (unsigned)(w >> 32);
+        key = min(key, nn_scan<ORDER, PREC>(rec(s0 + src, t), count(s0 + src, t), (unsigned)w, tpi,
+                                            lane, 32, irec));
+      }
+    }
+  }
+  // smallest key of the warp: ds2, then id
+  d = __reduce_min_sync(0xffffffffu, (unsigned)(key >> 32));
+  const unsigned id =
+      __reduce_min_sync(0xffffffffu, (unsigned)(key >> 32) == d ? (unsigned)key : ~0u);
+  if (lane < 12) {
+    if (lane == 10) acc = (double)__uint_as_float(d);
+    if (lane == 11) acc = (double)(int)id;
+    out[lane] = acc;
+  }
+}
+
 }  // namespace sapb
