@@ -294,7 +294,7 @@ int sapb_batch_run(sapb_batch *b, int flags) {
       e = cudaMemsetAsync(b->cnt_d, 0, sizeof(int) * (size_t)b->max_i, d->stream);
     if (e == cudaSuccess)
       e = launch_batch(d->order, d->prec, B, predict ? d->cap : 0, b->force_blocks, b->max_i,
-                       d->stream);
+                       d->num_sms, d->stream);
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(d->stream, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {

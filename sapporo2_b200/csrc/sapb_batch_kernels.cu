@@ -59,6 +59,8 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
   unsigned char *tiles = smem + kHdr;
   double *tot = reinterpret_cast<double *>(tiles + C::BODY);
   __shared__ int s_item;
+  Hits hits{reinterpret_cast<int2 *>(tiles + C::BODY + C::TOT_BYTES) + (threadIdx.x >> 5) * kHitBuf,
+            0};
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -194,20 +196,43 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
           }
           if (B.do_list)
             list_rescan_dp<C::RS>(Id[p], tmin[p] < Id[p].h2, gi[p], ty, tpi, rec, cnt, lane,
-                                  B.ngb_count, B.ngb_list);
+                                  hits, B.ngb_count, B.ngb_list);
         }
       } else {
         const float4 *rec = reinterpret_cast<const float4 *>(buf);
         const float2 z2 = make_float2(0.f, 0.f);
         AccMix2 Q{z2, z2, z2, z2, z2, z2, z2, z2, z2, z2};
         float2 tm = make_float2(FLT_MAX, FLT_MAX);
+        if (B.do_list) {
+          // 32 records of a row at a time: the list hits are one bit per record
+          // (all rows of the warp take every turn, some with no record left)
+          const int2 h2i = make_int2(list_radius(Im[0].h2), list_radius(Im[1].h2));
+#pragma unroll 1
+          for (int c0 = 0; c0 < cnt; c0 += 32 * tpi) {
+            const int k0 = c0 + ty, k1 = min(cnt, c0 + 32 * tpi);
+            uint2 hit = make_uint2(0u, 0u);
 #pragma unroll 2
-        for (int k = ty; k < cnt; k += tpi) {
-          const float4 r0 = rec[k * C::RS + 0];
-          const float4 r1 = rec[k * C::RS + 1];
-          const float4 r2 = rec[k * C::RS + 2];
-          const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
-          pair_mix2<ORDER>(I2, r0, r1, r2, r3, eps2v, Q, tm);
+            for (int k = k0; k < k1; k += tpi) {
+              const float4 r0 = rec[k * C::RS + 0];
+              const float4 r1 = rec[k * C::RS + 1];
+              const float4 r2 = rec[k * C::RS + 2];
+              const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
+              pair_mix2<ORDER, true>(I2, r0, r1, r2, r3, eps2v, Q, tm, hit, h2i);
+            }
+            const int n = rows_left(k0, k1, tpi);
+            hits_take<C::RS>(hits, hit.x, n, k0, tpi, rec, gi[0], lane, B.ngb_count, B.ngb_list);
+            hits_take<C::RS>(hits, hit.y, n, k0, tpi, rec, gi[1], lane, B.ngb_count, B.ngb_list);
+          }
+        } else {
+          uint2 none;
+#pragma unroll 2
+          for (int k = ty; k < cnt; k += tpi) {
+            const float4 r0 = rec[k * C::RS + 0];
+            const float4 r1 = rec[k * C::RS + 1];
+            const float4 r2 = rec[k * C::RS + 2];
+            const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
+            pair_mix2<ORDER>(I2, r0, r1, r2, r3, eps2v, Q, tm, none, int2{});
+          }
         }
         const float qv[2][10] = {
             {Q.ax.x, Q.ay.x, Q.az.x, -Q.pot.x, Q.jx.x, Q.jy.x, Q.jz.x, Q.sx.x, Q.sy.x, Q.sz.x},
@@ -233,9 +258,6 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
             best[p] = tmin[p];
             best_tile[p] = it;
           }
-          if (B.do_list)
-            list_rescan_mix<C::RS>(Im[p], tmin[p] < Im[p].h2, gi[p], ty, tpi, rec, cnt, lane,
-                                   B.ngb_count, B.ngb_list);
         }
       }
       __syncwarp();
@@ -303,34 +325,38 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
       }
     }
   }
+  if (B.do_list) hits_flush(hits, lane, B.ngb_count, B.ngb_list);
   if (broken && tid == 0) {
     for (int T = n_landed; T < n_issued; T++)
       mbar_wait_bounded(&full[T % C::NS], (uint32_t)((T / C::NS) & 1));
   }
 }
 
-// Sums the j-slices of every i and looks up its nearest neighbour's id: one
-// warp per i (reduce_one), a fixed grid striding over the active i.
-template <int ORDER, int PREC>
+// Sums the j-slices of every i and looks up its nearest neighbour's id: LPI
+// lanes per i (reduce_one), a fixed grid striding over the active i.
+template <int ORDER, int PREC, int LPI>
 __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs B) {
   constexpr int REC = PREC == DOUBLE ? 32 * pred_fields64(ORDER) : 16 * pred_fields(ORDER);
+  constexpr int PW = 32 / LPI;  // i per warp
   const BatchParams &P = *B.par;
   const int lane = threadIdx.x & 31;
   const unsigned char *pred = reinterpret_cast<const unsigned char *>(B.pred);
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < P.total_i;
-       i += (gridDim.x * blockDim.x) >> 5) {
-    const int c =
-        find_cluster(B.cl, P.n_clusters, i, [](const BatchCluster &q) { return q.i_first; });
-    if (c < 0) continue;
-    const BatchCluster &CL = B.cl[c];
-    if (i >= CL.i_first + CL.i_count) continue;
+  for (int i0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PW; i0 < P.total_i;
+       i0 += (int)((gridDim.x * blockDim.x) >> 5) * PW) {
+    const int i = i0 + lane / LPI;
+    const int c = i < P.total_i ? find_cluster(B.cl, P.n_clusters, i, [](const BatchCluster &q) {
+      return q.i_first;
+    }) : -1;
+    const BatchCluster &CL = B.cl[max(c, 0)];
+    const bool valid = c >= 0 && i < CL.i_first + CL.i_count;
     const int S = CL.nslices;
     const int sl = (CL.j_count + S - 1) / S;  // j per slice
-    double *out = B.res + (size_t)i * kResStride;
-    reduce_one<ORDER, PREC>(
-        S > 1 ? B.part + ((size_t)CL.part_base + (i - CL.i_first)) * kResStride : out,
-        (size_t)CL.i_count * kResStride, S, CL.tpi, lane, B.irec + (size_t)i * i_stride(ORDER),
-        out,
+    double *out = B.res + (size_t)(valid ? i : 0) * kResStride;
+    reduce_one<ORDER, PREC, LPI>(
+        valid,
+        valid && S > 1 ? B.part + ((size_t)CL.part_base + (i - CL.i_first)) * kResStride : out,
+        (size_t)CL.i_count * kResStride, S, CL.tpi, lane,
+        B.irec + (size_t)(valid ? i : 0) * i_stride(ORDER), out,
         [&](int s, unsigned t) { return pred + (size_t)(CL.j_first + s * sl + (int)t * kTJ) * REC; },
         [&](int s, unsigned t) {
           return min(kTJ, min(sl, CL.j_count - s * sl) - (int)t * kTJ);
@@ -341,7 +367,7 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs B) {
 // ---------------------------------------------------------------- launchers
 template <int ORDER, int PREC>
 static cudaError_t launch_batch_t(const BatchArgs &B, int j_grid, int force_blocks, int i_grid,
-                                  cudaStream_t st) {
+                                  int sms, cudaStream_t st) {
   using C = FCfg<ORDER, PREC, 2, 2>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -353,22 +379,24 @@ static cudaError_t launch_batch_t(const BatchArgs &B, int j_grid, int force_bloc
   if (B.do_predict && j_grid > 0)
     batch_predict_kernel<ORDER, PREC><<<(j_grid + 255) / 256, 256, 0, st>>>(B);
   batch_force_kernel<ORDER, PREC><<<force_blocks, kBT, C::SMEM, st>>>(B);
-  if (i_grid > 0)
-    batch_reduce_kernel<ORDER, PREC><<<std::min((i_grid + 7) / 8, 4 * force_blocks), 256, 0, st>>>(B);
+  if (i_grid > 0 && reduce_lanes(i_grid, sms) == 32)
+    batch_reduce_kernel<ORDER, PREC, 32><<<(i_grid + 7) / 8, 256, 0, st>>>(B);
+  else if (i_grid > 0)
+    batch_reduce_kernel<ORDER, PREC, 8><<<std::min((i_grid + 31) / 32, 8 * sms), 256, 0, st>>>(B);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch(int order, int prec, const BatchArgs &B, int j_grid, int force_blocks,
-                         int i_grid, cudaStream_t st) {
+                         int i_grid, int sms, cudaStream_t st) {
   if (order == GRAPE5) order = FOURTH;  // GRAPE-5 batches run the 4th-order kernels
   if (order == FOURTH && prec == DOUBLESINGLE)
-    return launch_batch_t<FOURTH, DOUBLESINGLE>(B, j_grid, force_blocks, i_grid, st);
+    return launch_batch_t<FOURTH, DOUBLESINGLE>(B, j_grid, force_blocks, i_grid, sms, st);
   if (order == FOURTH && prec == DOUBLE)
-    return launch_batch_t<FOURTH, DOUBLE>(B, j_grid, force_blocks, i_grid, st);
+    return launch_batch_t<FOURTH, DOUBLE>(B, j_grid, force_blocks, i_grid, sms, st);
   if (order == SIXTH && prec == DOUBLESINGLE)
-    return launch_batch_t<SIXTH, DOUBLESINGLE>(B, j_grid, force_blocks, i_grid, st);
+    return launch_batch_t<SIXTH, DOUBLESINGLE>(B, j_grid, force_blocks, i_grid, sms, st);
   if (order == SIXTH && prec == DOUBLE)
-    return launch_batch_t<SIXTH, DOUBLE>(B, j_grid, force_blocks, i_grid, st);
+    return launch_batch_t<SIXTH, DOUBLE>(B, j_grid, force_blocks, i_grid, sms, st);
   return cudaErrorInvalidValue;
 }
 

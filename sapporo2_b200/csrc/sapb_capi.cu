@@ -238,7 +238,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj) {
   // the balance between force and reduction depends on them
   const double sm_rate = d->prec == DOUBLE ? (d->order >= SIXTH ? 1.5e9 : 2.3e9)
                                            : (d->order >= SIXTH ? 3.6e9 : 5.6e9);
-  const int max_ns = std::max(1, ntiles / 4);  // keep >= 4 tiles per slice
+  const int max_ns = d->nslices ? ntiles : std::max(1, ntiles / 4);  // keep >= 4 tiles per slice
   // Mixed precision below 2^32 pairs and 2^19 j: the shape family comes from
   // the call size, the model above then picks the shape within it and the
   // j-split.  B200 sweeps of every shape and j-split (4th and 6th order, 256
@@ -595,6 +595,15 @@ static float near_r2(const sapb_dev *d, double eps2) {
   return (float)(d->near_k * eps2);
 }
 
+// Lists from one bit per record (two ALU operations per pair, gathered per 32
+// records) instead of rescans of the tiles that hold a neighbour: the bits win
+// where a tile holds neighbours of many of a warp's i, i.e. with few j in
+// address order (B200, about 32 neighbours: 16384 x 16384, 4th order, 437 us
+// against 530, and 390 without lists), and lose where few do (16384 i on
+// 131072 j, 6th order, 4.51 ms against 4.44) or where the spatial order puts a
+// warp's neighbours into a few tiles (8192 i on 131072 j 2.21 against 2.15).
+constexpr int kListBitsMaxJ = 65536;
+
 static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double eps2, int flags,
                      double *res_dev, int *cnt_dev, int *list_dev) {
   if (nj <= 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
@@ -625,6 +634,7 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
   A.nslices = P.ns;
   A.i_tiles = P.i_tiles;
   A.do_list = list ? 1 : 0;
+  A.list_bits = list && !spatial && d->prec != DOUBLE && nj < kListBitsMaxJ;
   A.ngb_count = cnt_dev;
   A.ngb_list = list_dev;
   A.status = d->status_d;
@@ -637,7 +647,7 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
   }
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
   const ReduceArgs R{A.out, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, A.iperm};
-  CK(d, launch_reduce(d->order, d->prec, R, d->stream));
+  CK(d, launch_reduce(d->order, d->prec, R, d->num_sms, d->stream));
   return SAPB_OK;
 }
 
@@ -762,13 +772,14 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
   A.nslices = P.ns;
   A.i_tiles = P.i_tiles;
   A.do_list = list ? 1 : 0;
+  A.list_bits = list && d->prec != DOUBLE && nj < kListBitsMaxJ;
   A.ngb_count = ngb_count_dev;
   A.ngb_list = ngb_list_dev;
   A.status = d->status_d;
   A.out = scratch;  // every (slice, valid i) record is written before it is read
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
   const ReduceArgs R{scratch, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, nullptr};
-  CK(d, launch_reduce(d->order, d->prec, R, d->stream));
+  CK(d, launch_reduce(d->order, d->prec, R, d->num_sms, d->stream));
   return SAPB_OK;
 }
 

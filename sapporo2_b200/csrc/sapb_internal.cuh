@@ -69,6 +69,7 @@ struct ForceArgs {
   int i_tiles;        // number of i tiles
   double *out;        // one 12-double record per (slice, i), see ReduceArgs
   int do_list;        // build neighbour lists
+  int list_bits;      // ... from one bit per record (mixed precision, address order)
   int *ngb_count;     // [ni] (zeroed before launch)
   int *ngb_list;      // [ni * 256]
   int *status;        // device error word

@@ -123,10 +123,12 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // with a huge value, which makes ds2 ~ 1e36 (1e300 in FP64): its force
 // underflows to zero and it can be neither nearest neighbour nor listed.
 //
-// Nearest neighbour and neighbour list cost one FMNMX per pair: the pair
-// loop only keeps the tile's minimum ds2.  Neighbour list: when that minimum
-// is below h2, the warp rescans the tile cooperatively (lanes split the j)
-// and appends the hits.  Nearest neighbour: each thread remembers the tile
+// Nearest neighbour: one FMNMX per pair, the pair loop only keeps the tile's
+// minimum ds2.  Neighbour list: the warp rescans a tile cooperatively (lanes
+// split the j) for each i whose h2 that minimum (on far tiles the box) comes
+// below; or, in mixed calls where most tiles hold neighbours (list_bits), two
+// more ALU operations per pair keep one bit per record and the warp gathers
+// the set bits after every 32 records.  Nearest neighbour: each thread remembers the tile
 // where its smallest ds2 first appeared, and the reduction looks up the id
 // there (reduce_one).  Rescans recompute ds2 bit-identically (same rounded
 // operations).
@@ -246,9 +248,13 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
   const float2 eps2v = make_float2(eps2f, eps2f);
   constexpr int NPAIR = IP / 2;  // packed i pairs per thread (mixed precision)
   IMix2 I2[NPAIR > 0 ? NPAIR : 1];
+  int2 h2i[NPAIR > 0 ? NPAIR : 1];
   if (PREC != DOUBLE) {
 #pragma unroll
-    for (int q = 0; q < NPAIR; q++) I2[q] = pack_i2(Im[2 * q], Im[(2 * q + 1) % IP]);
+    for (int q = 0; q < NPAIR; q++) {
+      I2[q] = pack_i2(Im[2 * q], Im[(2 * q + 1) % IP]);
+      h2i[q] = make_int2(list_radius(Im[2 * q].h2), list_radius(Im[(2 * q + 1) % IP].h2));
+    }
   }
 
   // ---- spatial mode: what a far tile must stay clear of, per i ----
@@ -276,6 +282,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
   const float shrink = spatial ? fminf(0.9999f, 1.f - 8.f * (0x1p-23f / A.far_c)) : 1.f;
   bool broken = false;
   int nfar = 0;  // far tiles of this warp (spatial mode)
+  Hits hits{reinterpret_cast<int2 *>(tiles + C::BODY + C::TOT_BYTES) + (tid >> 5) * kHitBuf, 0};
 
   for (int it = 0; it < nt; it++) {
     const int s = it % C::NS;
@@ -313,7 +320,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
         }
         if (A.do_list)
           list_rescan_dp<C::RS>(Id[p], tmin[p] < Id[p].h2, oi[p], ty, TPI, rec, cnt, lane,
-                                A.ngb_count, A.ngb_list);
+                                hits, A.ngb_count, A.ngb_list);
       }
     } else {
       const float4 *rec = reinterpret_cast<const float4 *>(buf);
@@ -376,7 +383,36 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
 #pragma unroll
             for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
           }
+        } else if (ORDER != GRAPE5 && A.list_bits) {
+          // 32 records of a row at a time: the list hits are one bit per record
+          // (all rows of the warp take every turn, some with no record left)
+#pragma unroll 1
+          for (int c0 = 0; c0 < cnt; c0 += 32 * TPI) {
+            const int k0 = c0 + ty, k1 = min(cnt, c0 + 32 * TPI);
+            uint2 hit[NPAIR];
+#pragma unroll
+            for (int q = 0; q < NPAIR; q++) hit[q] = make_uint2(0u, 0u);
+            SAPB_UNROLL(SAPB_JUNROLL)
+            for (int k = k0; k < k1; k += TPI) {
+              const float4 r0 = rec[k * C::RS + 0];
+              const float4 r1 = rec[k * C::RS + 1];
+              const float4 r2 = rec[k * C::RS + 2];
+              const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
+#pragma unroll
+              for (int q = 0; q < NPAIR; q++)
+                pair_mix2<ORDER, true>(I2[q], r0, r1, r2, r3, eps2v, Q[q], tm[q], hit[q], h2i[q]);
+            }
+            const int n = rows_left(k0, k1, TPI);
+#pragma unroll
+            for (int q = 0; q < NPAIR; q++) {
+              hits_take<C::RS>(hits, hit[q].x, n, k0, TPI, rec, oi[2 * q], lane, A.ngb_count,
+                               A.ngb_list);
+              hits_take<C::RS>(hits, hit[q].y, n, k0, TPI, rec, oi[(2 * q + 1) % IP], lane,
+                               A.ngb_count, A.ngb_list);
+            }
+          }
         } else {
+          uint2 none;
           SAPB_UNROLL(SAPB_JUNROLL)
           for (int k = ty; k < cnt; k += TPI) {
             const float4 r0 = rec[k * C::RS + 0];
@@ -385,7 +421,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
             const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
 #pragma unroll
             for (int q = 0; q < NPAIR; q++)
-              pair_mix2<ORDER>(I2[q], r0, r1, r2, r3, eps2v, Q[q], tm[q]);
+              pair_mix2<ORDER>(I2[q], r0, r1, r2, r3, eps2v, Q[q], tm[q], none, int2{});
           }
         }
 #pragma unroll
@@ -398,15 +434,34 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           tmin[2 * q + 1] = tm[q].y;
         }
       } else {
+        static_assert(IP % 2 == 0 || IP == 1, "one i or packed pairs per thread");
+        if (ORDER != GRAPE5 && A.list_bits) {
+          const int h2 = list_radius(Im[0].h2);
+#pragma unroll 1
+          for (int c0 = 0; c0 < cnt; c0 += 32 * TPI) {
+            const int k0 = c0 + ty, k1 = min(cnt, c0 + 32 * TPI);
+            unsigned hit = 0;
 #pragma unroll 2
-        for (int k = ty; k < cnt; k += TPI) {
-          const float4 r0 = rec[k * C::RS + 0];
-          const float4 r1 = rec[k * C::RS + 1];
-          const float4 r2 = rec[k * C::RS + 2];
-          const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
-#pragma unroll
-          for (int p = 0; p < IP; p++)
-            pair_mix<ORDER>(Im[p], r0, r1, r2, r3, eps2f, P[p], tmin[p]);
+            for (int k = k0; k < k1; k += TPI) {
+              const float4 r0 = rec[k * C::RS + 0];
+              const float4 r1 = rec[k * C::RS + 1];
+              const float4 r2 = rec[k * C::RS + 2];
+              const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
+              pair_mix<ORDER, true>(Im[0], r0, r1, r2, r3, eps2f, P[0], tmin[0], hit, h2);
+            }
+            hits_take<C::RS>(hits, hit, rows_left(k0, k1, TPI), k0, TPI, rec, oi[0], lane,
+                             A.ngb_count, A.ngb_list);
+          }
+        } else {
+          unsigned none;
+#pragma unroll 2
+          for (int k = ty; k < cnt; k += TPI) {
+            const float4 r0 = rec[k * C::RS + 0];
+            const float4 r1 = rec[k * C::RS + 1];
+            const float4 r2 = rec[k * C::RS + 2];
+            const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
+            pair_mix<ORDER>(Im[0], r0, r1, r2, r3, eps2f, P[0], tmin[0], none, 0);
+          }
         }
       }
 #pragma unroll
@@ -453,9 +508,9 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           // far tiles: no pair is closer than the tile's box, whose squared
           // distance from the high parts is, less the margin of the far test,
           // below the exact ds2 of every pair (lmask); the rescan itself is exact
-          if (A.do_list)
+          if (A.do_list && !A.list_bits)
             list_rescan_mix<C::RS>(Im[p], far ? ((lmask >> p) & 1u) != 0 : tmin[p] < Im[p].h2,
-                                   oi[p], ty, TPI, rec, cnt, lane, A.ngb_count, A.ngb_list);
+                                   oi[p], ty, TPI, rec, cnt, lane, hits, A.ngb_count, A.ngb_list);
         }
       }
     }
@@ -472,6 +527,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
       }
     }
   }
+  if (ORDER != GRAPE5 && A.do_list) hits_flush(hits, lane, A.ngb_count, A.ngb_list);
   if (spatial && A.stats && lane == 0) {
     atomicAdd(A.stats, (unsigned long long)nfar);
     atomicAdd(A.stats + 1, (unsigned long long)nt);
@@ -569,20 +625,20 @@ cudaError_t launch_wait_selftest(uint64_t limit_ns, int *status, cudaStream_t st
 }
 
 // ========================================================================
-// Reduction over the slices, and the nearest neighbour's id: one warp per i
+// Reduction over the slices, and the nearest neighbour's id: LPI lanes per i
 // (reduce_one).  With one slice `part` is `out`.
 // ========================================================================
-template <int ORDER, int PREC>
+template <int ORDER, int PREC, int LPI>
 __global__ void __launch_bounds__(256) reduce_kernel(ReduceArgs R) {
   constexpr int REC = PREC == DOUBLE ? 32 * pred_fields64(ORDER) : 16 * pred_fields(ORDER);
-  const int g = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (g >= R.ni) return;
-  const int i = R.iperm ? __ldg(R.iperm + g) : g;  // spatial mode: neighbours scan the same tiles
+  const int g = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) / LPI);
+  const bool valid = g < R.ni;
+  int i = valid ? g : 0;
+  if (valid && R.iperm) i = __ldg(R.iperm + g);  // spatial mode: neighbours scan the same tiles
   const unsigned char *pred = reinterpret_cast<const unsigned char *>(R.pred);
-  reduce_one<ORDER, PREC>(
-      R.part + (size_t)i * kResStride, (size_t)R.ni * kResStride, R.nslices, R.tpi, lane,
-      R.irec + (size_t)i * i_stride(ORDER), R.out + (size_t)i * kResStride,
+  reduce_one<ORDER, PREC, LPI>(
+      valid, R.part + (size_t)i * kResStride, (size_t)R.ni * kResStride, R.nslices, R.tpi,
+      threadIdx.x & 31, R.irec + (size_t)i * i_stride(ORDER), R.out + (size_t)i * kResStride,
       [&](int, unsigned t) { return pred + (size_t)t * kTJ * REC; },
       [&](int, unsigned t) { return min(kTJ, R.nj - (int)t * kTJ); });
 }
@@ -746,19 +802,22 @@ cudaError_t launch_readj(int order, int first, int n, double ti, int predict, co
 }
 
 template <int ORDER, int PREC>
-static cudaError_t launch_reduce_t(const ReduceArgs &R, cudaStream_t st) {
+static cudaError_t launch_reduce_t(const ReduceArgs &R, int sms, cudaStream_t st) {
   if (R.ni <= 0) return cudaSuccess;
-  reduce_kernel<ORDER, PREC><<<(R.ni + 7) / 8, 256, 0, st>>>(R);
+  if (reduce_lanes(R.ni, sms) == 32)
+    reduce_kernel<ORDER, PREC, 32><<<(R.ni + 7) / 8, 256, 0, st>>>(R);
+  else
+    reduce_kernel<ORDER, PREC, 8><<<(R.ni + 31) / 32, 256, 0, st>>>(R);
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, cudaStream_t st) {
-  if (order == GRAPE5 && prec == DOUBLESINGLE) return launch_reduce_t<GRAPE5, DOUBLESINGLE>(R, st);
+cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, int sms, cudaStream_t st) {
+  if (order == GRAPE5 && prec == DOUBLESINGLE) return launch_reduce_t<GRAPE5, DOUBLESINGLE>(R, sms, st);
   if (order == GRAPE5) order = FOURTH;  // as the force kernels
-  if (order == FOURTH && prec == DOUBLESINGLE) return launch_reduce_t<FOURTH, DOUBLESINGLE>(R, st);
-  if (order == FOURTH && prec == DOUBLE) return launch_reduce_t<FOURTH, DOUBLE>(R, st);
-  if (order == SIXTH && prec == DOUBLESINGLE) return launch_reduce_t<SIXTH, DOUBLESINGLE>(R, st);
-  if (order == SIXTH && prec == DOUBLE) return launch_reduce_t<SIXTH, DOUBLE>(R, st);
+  if (order == FOURTH && prec == DOUBLESINGLE) return launch_reduce_t<FOURTH, DOUBLESINGLE>(R, sms, st);
+  if (order == FOURTH && prec == DOUBLE) return launch_reduce_t<FOURTH, DOUBLE>(R, sms, st);
+  if (order == SIXTH && prec == DOUBLESINGLE) return launch_reduce_t<SIXTH, DOUBLESINGLE>(R, sms, st);
+  if (order == SIXTH && prec == DOUBLE) return launch_reduce_t<SIXTH, DOUBLE>(R, sms, st);
   return cudaErrorInvalidValue;
 }
 

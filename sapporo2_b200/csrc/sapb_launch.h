@@ -10,7 +10,7 @@ cudaError_t launch_predict(int order, int prec, int nj, double ti, const JState 
                            cudaStream_t st);
 cudaError_t launch_force(int order, int prec, const ForceArgs &A, int tpi, int ip,
                          cudaStream_t st);
-cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, cudaStream_t st);
+cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, int sms, cudaStream_t st);
 cudaError_t launch_wait_selftest(uint64_t limit_ns, int *status, cudaStream_t st);
 cudaError_t launch_readj(int order, int first, int n, double ti, int predict, const JState &js,
                          double *out, cudaStream_t st);
@@ -20,7 +20,7 @@ cudaError_t launch_readj(int order, int first, int n, double ti, int predict, co
 // capacities (j_grid threads, force_blocks blocks, i_grid threads) so the
 // launch sequence can be captured once in a CUDA graph.
 cudaError_t launch_batch(int order, int prec, const BatchArgs &B, int j_grid, int force_blocks,
-                         int i_grid, cudaStream_t st);
+                         int i_grid, int sms, cudaStream_t st);
 int batch_blocks_per_sm(int order, int prec);  // resident persistent blocks per SM
 
 int force_tile_i(int tpi, int ip);  // i-particles per block

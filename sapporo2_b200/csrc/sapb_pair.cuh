@@ -67,6 +67,8 @@ constexpr int kNS = 3;
 // (bytes 0..47) and, in spatial mode, the box of the tile in each stage
 // (2 float4 per stage, bytes 64..159); the tile ring starts at kHdr.
 constexpr int kHdr = 256;
+// Neighbour-list hits held per warp: written out above 32, one ballot adds up to 32.
+constexpr int kHitBuf = 64;
 
 template <int ORDER, int PREC, int TPI, int IP>
 struct FCfg {
@@ -86,7 +88,8 @@ struct FCfg {
   // i, [field][thread] so a warp's accesses are consecutive), which frees
   // 40 registers per thread and lets 4 blocks share an SM
   static constexpr int TOT_BYTES = PREC == DOUBLE ? 0 : IP * 10 * kBT * 8;
-  static constexpr int SMEM = kHdr + BODY + TOT_BYTES;
+  static constexpr int HIT_BYTES = kBT / 32 * kHitBuf * 8;  // neighbour-list hits, per warp
+  static constexpr int SMEM = kHdr + BODY + TOT_BYTES + HIT_BYTES;
   // resident blocks per SM the register budget is held to: FP64 kernels sit
   // at 168 registers, where one more allocation step (176) drops them from
   // 3 to 2 blocks per SM and costs 7 % at N = 2^20 (6th order)
@@ -124,10 +127,21 @@ __device__ __forceinline__ float pair_dr_mix(const IMix &I, const float4 &r0, co
   return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
-template <int ORDER>
+// Neighbour-list hits in the pair loop: one bit per record, shifted in from
+// the right: the sign of ds2 - h2 taken on their bits (both are >= 0, where
+// floats order as integers), an integer subtraction and a funnel shift on the
+// ALU pipe, which the FMA-bound loop leaves idle.
+__device__ __forceinline__ int list_radius(float h2) {  // no hits for h2 <= 0 and NaN
+  return h2 > 0.f ? __float_as_int(h2) : 0;
+}
+__device__ __forceinline__ void list_bit(unsigned &hit, float ds2, int h2) {
+  hit = __funnelshift_l((unsigned)(__float_as_int(ds2) - h2), hit, 1);
+}
+
+template <int ORDER, bool LIST = false>
 __device__ __forceinline__ void pair_mix(const IMix &I, const float4 &r0, const float4 &r1,
                                          const float4 &r2, const float4 &r3, float eps2,
-                                         AccMix &A, float &tmin) {
+                                         AccMix &A, float &tmin, unsigned &hit, int h2) {
   float dx, dy, dz, ds2;
   if (ORDER == GRAPE5) {  // every pair, the self pair included (kernels.cu:565)
     dx = ds_sub(r0.x, r1.x, I.xh, I.xl);
@@ -137,6 +151,7 @@ __device__ __forceinline__ void pair_mix(const IMix &I, const float4 &r0, const 
   } else {
     ds2 = pair_dr_mix(I, r0, r1, dx, dy, dz);
     tmin = fminf(tmin, ds2);
+    if (LIST) list_bit(hit, ds2, h2);
   }
   const float inv = rsqrt_mufu(ds2 + eps2);
   const float inv2 = inv * inv;
@@ -216,9 +231,10 @@ struct Pre2 {
 // ALU pipe): choosing an unmasked loop per tile from the tiles' id ranges
 // measured 2 % slower on B200, the two loop copies costing more than the
 // four ALU instructions they save.
-template <bool NGB = true>  // false (GRAPE-5): no self-pair mask, no nearest-neighbour minimum
+// NGB false (GRAPE-5): no self-pair mask, no nearest-neighbour minimum.
+template <bool NGB, bool LIST>
 __device__ __forceinline__ Pre2 pair_mix2_pre(const IMix2 &I, const float4 &r0, const float4 &r1,
-                                              float2 eps2, float2 &tmin) {
+                                              float2 eps2, float2 &tmin, uint2 &hit, int2 h2) {
   Pre2 P;
   // x - y == x + (-y) exactly, so these equal ds_sub of the scalar path
   P.dx = __fadd2_rn(__fadd2_rn(bc2(r0.x), I.nxh), __fadd2_rn(bc2(r1.x), I.nxl));
@@ -233,6 +249,10 @@ __device__ __forceinline__ Pre2 pair_mix2_pre(const IMix2 &I, const float4 &r0, 
   if (NGB) {
     tmin.x = fminf(tmin.x, ds2.x);
     tmin.y = fminf(tmin.y, ds2.y);
+  }
+  if (LIST) {
+    list_bit(hit.x, ds2.x, h2.x);
+    list_bit(hit.y, ds2.y, h2.y);
   }
   const float2 r2v = __fadd2_rn(ds2, eps2);
   P.inv = make_float2(rsqrt_mufu(r2v.x), rsqrt_mufu(r2v.y));
@@ -282,11 +302,11 @@ __device__ __forceinline__ void pair_mix2_post(const IMix2 &I, const Pre2 &P, fl
   }
 }
 
-template <int ORDER>
+template <int ORDER, bool LIST = false>
 __device__ __forceinline__ void pair_mix2(const IMix2 &I, const float4 &r0, const float4 &r1,
                                           const float4 &r2, const float4 &r3, float2 eps2,
-                                          AccMix2 &A, float2 &tmin) {
-  const Pre2 P = pair_mix2_pre<ORDER != GRAPE5>(I, r0, r1, eps2, tmin);
+                                          AccMix2 &A, float2 &tmin, uint2 &hit, int2 h2) {
+  const Pre2 P = pair_mix2_pre<ORDER != GRAPE5, LIST>(I, r0, r1, eps2, tmin, hit, h2);
   pair_mix2_post<ORDER>(I, P, r0.w, r2, r3, A);
 }
 
@@ -376,18 +396,64 @@ __device__ __forceinline__ void pair_dp(const IDp &I, const double4 &r0, const d
   }
 }
 
-__device__ __forceinline__ void list_push(int *cnt, int *list, int gi, int idj) {
-  const int pos = atomicAdd(cnt + gi, 1);
-  if (pos < kNgbPB) list[(size_t)gi * kNgbPB + pos] = idj;
+// Neighbour-list hits of one warp, gathered in shared memory and written to
+// the lists 33 to 64 at a time.  A hit takes a slot of its list with one
+// global atomic whose answer the store needs: taken where the hit is found,
+// the warp waits there for L2, hit after hit; here all lanes have one in
+// flight.
+struct Hits {
+  int2 *buf;  // {i, j's id}
+  int n;      // entries held (the same in every lane)
+};
+__device__ __forceinline__ void hits_flush(Hits &H, int lane, int *cnt, int *list) {
+  __syncwarp();
+  for (int e = lane; e < H.n; e += 32) {
+    const int2 v = H.buf[e];
+    const int pos = atomicAdd(cnt + v.x, 1);
+    if (pos < kNgbPB) list[(size_t)v.x * kNgbPB + pos] = v.y;
+  }
+  __syncwarp();
+  H.n = 0;
+}
+// One entry of every lane with `hit` set (called by the whole warp).
+__device__ __forceinline__ void hits_add(Hits &H, bool hit, int gi, int id, int lane, int *cnt,
+                                         int *list) {
+  const unsigned m = __ballot_sync(0xffffffffu, hit);
+  if (!m) return;
+  if (hit) H.buf[H.n + __popc(m & ((1u << lane) - 1u))] = make_int2(gi, id);
+  H.n += __popc(m);
+  if (H.n > kHitBuf - 32) hits_flush(H, lane, cnt, list);
+}
+
+// Records k0, k0 + tpi, ... below k1.
+__device__ __forceinline__ int rows_left(int k0, int k1, int tpi) {
+  return k0 < k1 ? (k1 - k0 + tpi - 1) / tpi : 0;
+}
+// Gathers the hits of up to 32 records: bit n - 1 - q of `hit` is record
+// k0 + q * tpi (called by the whole warp; n may differ between its rows).
+template <int RS>
+__device__ __forceinline__ void hits_take(Hits &H, unsigned hit, int n, int k0, int tpi,
+                                          const float4 *rec, int gi, int lane, int *cnt,
+                                          int *list) {
+  while (__any_sync(0xffffffffu, hit != 0)) {
+    const bool some = hit != 0;
+    int id = 0;
+    if (some) {
+      const int b = 31 - __clz(hit);
+      hit ^= 1u << b;
+      id = __float_as_int(rec[(k0 + (n - 1 - b) * tpi) * RS + 1].w);
+    }
+    hits_add(H, some, gi, id, lane, cnt, list);
+  }
 }
 
 // Warp-cooperative neighbour-list rescan of one shared-memory tile: for every
 // lane whose i saw a pair below h2 in this tile, the whole warp re-evaluates
-// that i against the tile's j (lane-strided) and appends the hits.
+// that i against the tile's j (lane-strided) and gathers the hits.
 template <int RS>
 __device__ __forceinline__ void list_rescan_mix(const IMix &I, bool want, int gi, int row,
                                                 int TPI, const float4 *rec, int cnt, int lane,
-                                                int *ngb_count, int *ngb_list) {
+                                                Hits &H, int *ngb_count, int *ngb_list) {
   unsigned m = __ballot_sync(0xffffffffu, want);
   while (m) {
     const int src = __ffs(m) - 1;
@@ -403,12 +469,18 @@ __device__ __forceinline__ void list_rescan_mix(const IMix &I, bool want, int gi
     S.id = __shfl_sync(0xffffffffu, I.id, src);
     const int sgi = __shfl_sync(0xffffffffu, gi, src);
     const int srow = __shfl_sync(0xffffffffu, row, src);
-    for (int k = srow + lane * TPI; k < cnt; k += 32 * TPI) {
-      float dx, dy, dz;
-      const float4 r0 = rec[k * RS + 0];
-      const float4 r1 = rec[k * RS + 1];
-      const float ds2 = pair_dr_mix(S, r0, r1, dx, dy, dz);
-      if (ds2 < S.h2) list_push(ngb_count, ngb_list, sgi, __float_as_int(r1.w));
+    for (int k0 = srow; k0 < cnt; k0 += 32 * TPI) {
+      const int k = k0 + lane * TPI;
+      bool hit = false;
+      int id = 0;
+      if (k < cnt) {
+        float dx, dy, dz;
+        const float4 r0 = rec[k * RS + 0];
+        const float4 r1 = rec[k * RS + 1];
+        hit = pair_dr_mix(S, r0, r1, dx, dy, dz) < S.h2;
+        id = __float_as_int(r1.w);
+      }
+      hits_add(H, hit, sgi, id, lane, ngb_count, ngb_list);
     }
   }
 }
@@ -500,7 +572,7 @@ __device__ __noinline__ void near_rescan_mix(unsigned nm, int oi, int row, int t
 template <int RS>
 __device__ __forceinline__ void list_rescan_dp(const IDp &I, bool want, int gi, int row,
                                                int TPI, const double4 *rec, int cnt, int lane,
-                                               int *ngb_count, int *ngb_list) {
+                                               Hits &H, int *ngb_count, int *ngb_list) {
   unsigned m = __ballot_sync(0xffffffffu, want);
   while (m) {
     const int src = __ffs(m) - 1;
@@ -513,16 +585,21 @@ __device__ __forceinline__ void list_rescan_dp(const IDp &I, bool want, int gi, 
     S.id = __shfl_sync(0xffffffffu, I.id, src);
     const int sgi = __shfl_sync(0xffffffffu, gi, src);
     const int srow = __shfl_sync(0xffffffffu, row, src);
-    for (int k = srow + lane * TPI; k < cnt; k += 32 * TPI) {
-      double dx, dy, dz;
-      const double4 r0 = rec[k * RS + 0];
-      const double4 r1 = rec[k * RS + 1];
-      const double ds2 = pair_dr_dp(S, r0, r1, dx, dy, dz);
-      if (ds2 < S.h2) list_push(ngb_count, ngb_list, sgi, __double2loint(r1.w));
+    for (int k0 = srow; k0 < cnt; k0 += 32 * TPI) {
+      const int k = k0 + lane * TPI;
+      bool hit = false;
+      int id = 0;
+      if (k < cnt) {
+        double dx, dy, dz;
+        const double4 r0 = rec[k * RS + 0];
+        const double4 r1 = rec[k * RS + 1];
+        hit = pair_dr_dp(S, r0, r1, dx, dy, dz) < S.h2;
+        id = __double2loint(r1.w);
+      }
+      hits_add(H, hit, sgi, id, lane, ngb_count, ngb_list);
     }
   }
 }
-
 
 // ---------------- nearest neighbour ----------------
 // The pair loops keep, per thread and i, only the smallest ds2 and the tile
@@ -632,67 +709,101 @@ __device__ __forceinline__ void nn_rows(int tpi, Row row, Rec rec, Count count,
   }
 }
 
-// One i's records, one per slice, `step` doubles apart, summed by one warp:
-// lanes 0..9 and 16..25 sum one field each over the even and the odd slices
-// (fixed order, so results are bit-stable); one lane per slice finds the
-// smallest ds2, and the whole warp scans the tile it was seen in, eight
-// records per lane, for the id.  Small calls are bound by latency (one thread
-// per i used to walk slices x 12 words in a row; 48 i on 16384 j, 16 slices,
-// predictor and force included: 37.0 -> 32.2 us on B200), large ones by L2.
-// `part` may be `out`: the warp has read its records before it writes.
+// One i's records, one per slice, `step` doubles apart, summed by a group of
+// LPI lanes: every eight lanes take one record at a time, two words per lane,
+// lanes 0..4 the sums and lane 5 the nearest neighbour's words; with LPI = 32
+// four records are under way at once (fixed order either way, so results are
+// bit-stable).  Then the whole group scans the tile that saw the smallest ds2
+// for its id.  LPI = 32 is for calls with too few i to fill the GPU, which are
+// bound by the latency of the chain (one thread per i, walking slices x 12
+// words in a row: 48 i on 16384 j 117 us a pass, a warp per i 105); more i are
+// bound by the loads, and a warp each makes a second wave of warps of it
+// (16384 i x 2 slices, passes back to back 336 us; eight lanes each 332).
+// All lanes of the warp call this; `part` may be `out`.
 // `rec(s, t)` / `count(s, t)`: records of tile t as slice s numbers them.
-template <int ORDER, int PREC, typename Rec, typename Count>
-__device__ __forceinline__ void reduce_one(const double *part, size_t step, int nslices, int tpi,
-                                           int lane, const double *irec, double *out, Rec rec,
-                                           Count count) {
-  const int f = lane & 15;
-  double acc = 0.0;
-  if (f < 10) {
-#pragma unroll 4
-    for (int s = lane >> 4; s < nslices; s += 2) acc += part[s * step + f];
-  }
-  acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-
+template <int ORDER, int PREC, int LPI, typename Rec, typename Count>
+__device__ __forceinline__ void reduce_one(bool valid, const double *part, size_t step,
+                                           int nslices, int tpi, int lane, const double *irec,
+                                           double *out, Rec rec, Count count) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int f = lane & 7, sub = (lane & (LPI - 1)) >> 3;
   const unsigned none = __float_as_uint(kNoNgbDs2);
-  unsigned d = none;
-  if (ORDER != GRAPE5)
-    for (int s = lane; s < nslices; s += 32)
-      d = min(d, (unsigned)__double2hiint(part[s * step + 10]));
-  d = __reduce_min_sync(0xffffffffu, d);
-  unsigned long long key = nn_key(kNoNgbDs2, -1);
-  if (d != none) {
-    for (int s0 = 0; s0 < nslices; s0 += 32) {
-      unsigned long long where = kNnDone;
-      bool todo = false;
-      if (s0 + lane < nslices) {
-        const double *o = part + (s0 + lane) * step;
-        const unsigned long long k = (unsigned long long)__double_as_longlong(o[10]);
-        where = (unsigned long long)__double_as_longlong(o[11]);
-        if ((unsigned)(k >> 32) == d) {
-          todo = where != kNnDone;
-          if (!todo) key = min(key, k);
-        }
-      }
-      unsigned m = __ballot_sync(0xffffffffu, todo);
-      while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        const unsigned long long w = __shfl_sync(0xffffffffu, where, src);
-        const unsigned t = (unsigned)(w >> 32);
-        key = min(key, nn_scan<ORDER, PREC>(rec(s0 + src, t), count(s0 + src, t), (unsigned)w, tpi,
-                                            lane, 32, irec));
+  double ax = 0.0, ay = 0.0;
+  unsigned long long key = nn_key(kNoNgbDs2, -1), where = kNnDone;
+  int slice = 0, tie = 0;  // tie: slices saw the same ds2 and not all know the id
+  auto take = [&](unsigned long long k, unsigned long long w, int s) {
+    const unsigned d = (unsigned)(k >> 32), m = (unsigned)(key >> 32);
+    if (d < m) {
+      key = k; where = w; slice = s; tie = 0;
+    } else if (d == m && d != none) {
+      if ((w & where) == kNnDone) key = min(key, k);
+      else tie = 1;
+    }
+  };
+  if (valid && f < 6) {
+#pragma unroll 4
+    for (int s = sub; s < nslices; s += LPI / 8) {
+      const double x = part[s * step + 2 * f], y = part[s * step + 2 * f + 1];
+      ax += x;
+      ay += y;
+      if (ORDER != GRAPE5 && f == 5)
+        take((unsigned long long)__double_as_longlong(x),
+             (unsigned long long)__double_as_longlong(y), s);
+    }
+  }
+#pragma unroll
+  for (int o = 8; o < LPI; o <<= 1) {
+    ax += __shfl_xor_sync(kAll, ax, o);
+    ay += __shfl_xor_sync(kAll, ay, o);
+    const unsigned long long k = __shfl_xor_sync(kAll, key, o), w = __shfl_xor_sync(kAll, where, o);
+    const int s = __shfl_xor_sync(kAll, slice, o), t = __shfl_xor_sync(kAll, tie, o);
+    const bool same = (unsigned)(k >> 32) == (unsigned)(key >> 32);
+    const int had = tie;
+    take(k, w, s);
+    if (same) tie |= had | t;
+    else if ((unsigned)(k >> 32) == (unsigned)(key >> 32)) tie = t;  // theirs was taken
+  }
+  const int src = (lane & ~(LPI - 1)) | 5;
+  key = __shfl_sync(kAll, key, src);
+  where = __shfl_sync(kAll, where, src);
+  slice = __shfl_sync(kAll, slice, src);
+  tie = __shfl_sync(kAll, tie, src);
+  const unsigned d = (unsigned)(key >> 32);
+  const int l = lane & (LPI - 1);
+  if (valid && d != none) {
+    if (!tie) {
+      if (where != kNnDone)
+        key = nn_scan<ORDER, PREC>(rec(slice, (unsigned)(where >> 32)),
+                                   count(slice, (unsigned)(where >> 32)), (unsigned)where, tpi, l,
+                                   LPI, irec);
+    } else {
+      key = nn_key(kNoNgbDs2, -1);
+      for (int s = 0; s < nslices; s++) {
+        const unsigned long long k = (unsigned long long)__double_as_longlong(part[s * step + 10]);
+        const unsigned long long w = (unsigned long long)__double_as_longlong(part[s * step + 11]);
+        if ((unsigned)(k >> 32) != d) continue;
+        key = min(key, w == kNnDone
+                           ? k
+                           : nn_scan<ORDER, PREC>(rec(s, (unsigned)(w >> 32)),
+                                                  count(s, (unsigned)(w >> 32)), (unsigned)w, tpi, l,
+                                                  LPI, irec));
       }
     }
   }
-  // smallest key of the warp: ds2, then id
-  d = __reduce_min_sync(0xffffffffu, (unsigned)(key >> 32));
-  const unsigned id =
-      __reduce_min_sync(0xffffffffu, (unsigned)(key >> 32) == d ? (unsigned)key : ~0u);
-  if (lane < 12) {
-    if (lane == 10) acc = (double)__uint_as_float(d);
-    if (lane == 11) acc = (double)(int)id;
-    out[lane] = acc;
+#pragma unroll
+  for (int o = 1; o < LPI; o <<= 1) key = min(key, __shfl_xor_sync(kAll, key, o));
+  if (valid && l < 6) {
+    if (l == 5) {
+      ax = (double)__uint_as_float((unsigned)(key >> 32));
+      ay = (double)(int)(unsigned)key;
+    }
+    out[2 * l] = ax;
+    out[2 * l + 1] = ay;
   }
 }
+
+// Lanes per i of a reduction over `ni` i: a warp each while all are resident
+// together on `sms` SMs.
+inline int reduce_lanes(int ni, int sms) { return ni <= 64 * sms ? 32 : 8; }
 
 }  // namespace sapb
