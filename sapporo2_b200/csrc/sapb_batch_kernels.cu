@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
   using C = FCfg<ORDER, PREC, 2, 2>;  // shared-memory plan with a row reduction area
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *empty = full + C::NS;
+  Ring *ring = reinterpret_cast<Ring *>(smem + kRing);
   unsigned char *tiles = smem + kHdr;
   double *tot = reinterpret_cast<double *>(tiles + C::BODY);
   __shared__ int s_item;
@@ -69,19 +69,14 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
 
   if (tid == 0) {
 #pragma unroll
-    for (int s = 0; s < C::NS; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kBT / 32);
-    }
+    for (int s = 0; s < C::NS; s++) mbar_init(&full[s], 1);
+    *ring = Ring{};
     fence_barrier_init();
   }
   __syncthreads();
 
   int tbase = 0;  // tiles this block has streamed so far (ring position)
   bool broken = false;
-  // thread 0: ring positions issued / seen arrived; after a timed-out wait
-  // the copies in between are drained before the block exits
-  int n_issued = 0, n_landed = 0;
   for (;;) {
     if (tid == 0) s_item = atomicAdd(&B.par->queue_head, 1);
     __syncthreads();
@@ -144,33 +139,23 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
       const int st = T % C::NS;
       const int cnt = min(kTJ, W.j_count - t * kTJ);
       const uint32_t bytes = (uint32_t)(cnt * C::REC);
-      n_issued = T + 1;
+      ring->issued[st]++;
       fence_proxy_async();
       mbar_expect_tx(&full[st], bytes);
       bulk_g2s(tiles + st * C::TILE_BYTES, pred + (size_t)(W.j_begin + t * kTJ) * C::REC, bytes,
                &full[st]);
     };
-    if (tid == 0 && !broken) {
-      for (int t = 0; t < C::NS && t < nt; t++) {
-        const int T = tbase + t;
-        if (T >= C::NS &&
-            !mbar_wait_bounded(&empty[T % C::NS], (uint32_t)((T / C::NS - 1) & 1))) {
-          broken = true;
-          atomicOr(B.status, kErrWaitTimeout);
-          break;
-        }
-        issue(t);
-      }
-    }
+    // every warp is past the previous item's tiles (barriers above)
+    if (tid == 0 && ring->stop == 0)
+      for (int t = 0; t < C::NS && t < nt; t++) issue(t);
 
     for (int it = 0; it < nt; it++) {
       const int T = tbase + it;
       const int s = T % C::NS;
       if (!broken) {
-        if (mbar_wait_bounded(&full[s], (uint32_t)((T / C::NS) & 1))) {
-          n_landed = T + 1;
-        } else {
+        if (!mbar_wait_bounded(&full[s], (uint32_t)((T / C::NS) & 1))) {
           broken = true;
+          ring->stop = 1;  // no more copies: the stages' turn order is lost
           atomicOr(B.status, kErrWaitTimeout);
         }
       }
@@ -261,15 +246,7 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-      if (tid == 0 && !broken && it + C::NS < nt) {
-        if (mbar_wait_bounded(&empty[s], (uint32_t)((T / C::NS) & 1))) {
-          issue(it + C::NS);
-        } else {
-          broken = true;
-          atomicOr(B.status, kErrWaitTimeout);
-        }
-      }
+      if (lane == 0 && it + C::NS < nt && ring->last(s)) issue(it + C::NS);
     }
     tbase += nt;
 
@@ -326,10 +303,7 @@ __global__ void __launch_bounds__(kBT, (PREC == DOUBLE ? 1 : (ORDER >= SIXTH ? 3
     }
   }
   if (B.do_list) hits_flush(hits, lane, B.ngb_count, B.ngb_list);
-  if (broken && tid == 0) {
-    for (int T = n_landed; T < n_issued; T++)
-      mbar_wait_bounded(&full[T % C::NS], (uint32_t)((T / C::NS) & 1));
-  }
+  if (__syncthreads_or(broken) && tid == 0) ring_drain(full, *ring, C::NS);
 }
 
 // Sums the j-slices of every i and looks up its nearest neighbour's id: LPI

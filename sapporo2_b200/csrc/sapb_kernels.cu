@@ -108,9 +108,9 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // of TI = TIT*IP particles.  blockIdx.y selects j-slice s of S: the tiles
 // s, s+S, s+2S, ... of kTJ = 256 records.  Lane 0 of warp 0 streams them
 // into a 3-stage shared-memory ring with cp.async.bulk (TMA engine): `full`
-// mbarriers signal arrival (complete_tx), `empty` mbarriers collect one
-// arrival per warp; there is no block-wide barrier per tile, so warps drift
-// up to two tiles apart instead of waiting for the slowest one.
+// mbarriers signal arrival (complete_tx), and the warp that releases a stage
+// last refills it; there is no block-wide barrier per tile and no warp waits
+// for another one's release, so warps drift up to two tiles apart.
 // Row `ty` consumes records ty, ty+TPI, ... of each tile.
 //
 // Mixed precision (DOUBLESINGLE): dr = (xj_hi - xi_hi) + (xj_lo - xi_lo)
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
   using C = FCfg<ORDER, PREC, TPI, IP>;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *empty = full + C::NS;
+  Ring *ring = reinterpret_cast<Ring *>(smem + kRing);
   float4 *sbox = reinterpret_cast<float4 *>(smem + 64);  // spatial mode: box of each stage's tile
   unsigned char *tiles = smem + kHdr;
 
@@ -169,32 +169,25 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
 
   if (tid == 0) {
 #pragma unroll
-    for (int s = 0; s < C::NS; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kBT / 32);
-    }
+    for (int s = 0; s < C::NS; s++) mbar_init(&full[s], 1);
+    *ring = Ring{};
     fence_barrier_init();
   }
   __syncthreads();
 
-  // ---- producer: lane 0 of warp 0 fills the ring ----
-  // n_issued / n_landed (thread 0): tiles issued so far / tiles whose
-  // arrival it has seen; after a timed-out wait the copies in between are
-  // drained before the block exits
-  int n_issued = 0, n_landed = 0;
+  // ---- the ring: thread 0 fills it, then whoever releases a stage last ----
   auto issue = [&](int it) {
-    n_issued = it + 1;
     const int st = it % C::NS;
     const int tile = slice + it * S;
     const int cnt = min(kTJ, A.nj - tile * kTJ);
     const uint32_t bytes = (uint32_t)(cnt * C::REC);
+    ring->issued[st]++;
     fence_proxy_async();
     mbar_expect_tx(&full[st], bytes + (spatial ? 32u : 0u));
     bulk_g2s(tiles + st * C::TILE_BYTES, pred + (size_t)tile * kTJ * C::REC, bytes, &full[st]);
     if (spatial) bulk_g2s(sbox + 2 * st, A.tbox + 2 * tile, 32u, &full[st]);
   };
-  const bool producer = (tid == 0);
-  if (producer)
+  if (tid == 0)
     for (int it = 0; it < C::NS && it < nt; it++) issue(it);
 
   // ---- consumers: 128 threads = TPI rows x TIT columns, IP i each ----
@@ -287,10 +280,9 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
   for (int it = 0; it < nt; it++) {
     const int s = it % C::NS;
     if (!broken) {
-      if (mbar_wait_bounded(&full[s], (uint32_t)((it / C::NS) & 1))) {
-        n_landed = it + 1;
-      } else {
+      if (!mbar_wait_bounded(&full[s], (uint32_t)((it / C::NS) & 1))) {
         broken = true;
+        ring->stop = 1;  // no more copies: the stages' turn order is lost
         atomicOr(A.status, kErrWaitTimeout);
       }
     }
@@ -515,29 +507,15 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
       }
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);  // this warp is done with the stage
-    // Refill the stage once all four warps released it; only warp 0 waits
-    // here, the others may already be up to C::NS-1 tiles ahead.
-    if (producer && !broken && it + C::NS < nt) {
-      if (mbar_wait_bounded(&empty[s], (uint32_t)((it / C::NS) & 1))) {
-        issue(it + C::NS);
-      } else {
-        broken = true;
-        atomicOr(A.status, kErrWaitTimeout);
-      }
-    }
+    if (lane == 0 && it + C::NS < nt && ring->last(s)) issue(it + C::NS);
   }
   if (ORDER != GRAPE5 && A.do_list) hits_flush(hits, lane, A.ngb_count, A.ngb_list);
   if (spatial && A.stats && lane == 0) {
     atomicAdd(A.stats, (unsigned long long)nfar);
     atomicAdd(A.stats + 1, (unsigned long long)nt);
   }
-  if (broken && producer) {
-    // let the copies still in flight land (bounded waits) before the block
-    // exits and its shared memory is released
-    for (int it = n_landed; it < n_issued; it++)
-      mbar_wait_bounded(&full[it % C::NS], (uint32_t)((it / C::NS) & 1));
-  }
+  // all warps are past their last tile
+  if (__syncthreads_or(broken) && tid == 0) ring_drain(full, *ring, C::NS);
 
   if (PREC != DOUBLE) {
 #pragma unroll
@@ -553,7 +531,6 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
   auto tile_rec = [&](unsigned t) { return pred + (size_t)t * kTJ * C::REC; };
   auto tile_cnt = [&](unsigned t) { return min(kTJ, A.nj - (int)t * kTJ); };
   if (TPI > 1) {
-    named_barrier(1, kBT);  // all consumer warps are past their last tile
     double *red = reinterpret_cast<double *>(tiles);
 #pragma unroll
     for (int p = 0; p < IP; p++) {

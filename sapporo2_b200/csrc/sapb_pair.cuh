@@ -63,10 +63,41 @@ __device__ __forceinline__ void taylor(const JState &js, int k, double ti, doubl
 constexpr int kBT = 128;
 constexpr int kTJ = 256;
 constexpr int kNS = 3;
-// Shared-memory header of the force kernel: full/empty mbarriers of the ring
-// (bytes 0..47) and, in spatial mode, the box of the tile in each stage
-// (2 float4 per stage, bytes 64..159); the tile ring starts at kHdr.
+// Shared-memory header of the force kernel: full mbarriers of the ring
+// (bytes 0..23), in spatial mode the box of the tile in each stage (2 float4
+// per stage, bytes 64..159), and the ring's counters (from byte 160); the
+// tile ring starts at kHdr.
 constexpr int kHdr = 256;
+constexpr int kRing = 160;
+
+// The warp that releases a stage last refills it at once.  (One lane of warp
+// 0 used to wait for the other warps at every tile and then refill: its warp
+// computed in step with the slowest.  B200, a pass: 12983 i on 131072 j, where
+// warps differ by their near tiles and lists, 4.19 -> 4.09 ms; 192-cluster
+// batch 2.65 -> 2.58; calls whose warps are alike unchanged within 0.5 %.)
+struct Ring {
+  unsigned left[kNS];    // warps that have released the stage's present tile
+  unsigned issued[kNS];  // copies issued into the stage
+  unsigned stop;         // a wait timed out
+
+  // Called by one lane of each warp, after the warp's last read of stage s:
+  // true for the last of them, unless the ring has stopped.
+  __device__ __forceinline__ bool last(int s) {
+    __threadfence_block();
+    if (atomicAdd(&left[s], 1u) != kBT / 32 - 1) return false;
+    __threadfence_block();
+    left[s] = 0;
+    return *(volatile unsigned *)&stop == 0;
+  }
+};
+static_assert(kRing + sizeof(Ring) <= kHdr, "header");
+
+// After a timed-out wait: lets the copies still in flight land (bounded
+// waits) before the block exits and its shared memory is released.
+__device__ __forceinline__ void ring_drain(uint64_t *full, const Ring &r, int stages) {
+  for (int s = 0; s < stages; s++)
+    if (r.issued[s]) mbar_wait_bounded(&full[s], (r.issued[s] - 1) & 1);
+}
 // Neighbour-list hits held per warp: written out above 32, one ballot adds up to 32.
 constexpr int kHitBuf = 64;
 
