@@ -5,6 +5,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <math.h>
+
 #include <algorithm>
 #include <climits>
 #include <new>
@@ -208,121 +210,123 @@ static int blocks_per_sm(int order, int prec, int tpi, int ip) {
   return std::max(1, force_blocks_per_sm(order, prec, tpi, ip));
 }
 
-// Launch shape for ni i-particles and nj j: threads-per-i, i per thread and
-// the number of j-slices S.  Cost model: blocks of one shape run in waves
-// of R = SMs x resident blocks per SM; a block of st tiles costs
-// (st + 1) tile-times (prologue, nearest-neighbour rescan, epilogue), a
-// tile-time being 128 x (i per block) x (blocks per SM) pair-times of one
-// SM; S > 1 adds the slice reduction (S x ni records read).  The block
-// count B = i-tiles x S is chosen near a whole number of waves: a last wave
-// that holds a few blocks costs as much as a full one.
+// Launch shape for ni i-particles and nj j.
+//
+// Threads per i and i per thread come from the call's size (shape_family,
+// from sweeps of every shape and j-split on B200); where two are given the
+// cost below decides.  The number of j-slices S minimises the cost of
+// B = i-tiles x S blocks in R = SMs x resident blocks slots: a block costs
+// its tiles plus kBlockTiles for its start and end; up to one wave the call
+// takes as long as its longest block, beyond that as long as the slots take
+// for all blocks, plus kTail of the part of the last wave that stays empty.
+// With a share u of an SM's slots in use a tile takes sqrt(u) of its time on
+// a full SM (latency, not the pipe, bounds a block there).  Each slice adds
+// its records to the reduction, and kSliceS to that kernel's chain of loads.
+// Over 130 calls of 4 to 16384 i on 1024 to 131072 j, lists on, the plans are
+// within 2.4 % of the best of the sweep on average; the previous ones (whole
+// waves, a tile for every block's start, four tiles or more per slice, larger
+// shapes) within 8 to 12 %.
+constexpr double kBlockTiles = 0.3, kTail = 0.6, kSliceS = 5e-8;
 extern "C" {
 static bool use_spatial(const sapb_dev *d, int ni, int nj);  // defined with the C ABI below
+}
+
+struct Shape {
+  int tpi, ip;
+  double eff;  // throughput of a full GPU relative to the others of its family
+};
+
+static int shape_family(const sapb_dev *d, int ni, int nj, Shape out[2]) {
+  auto one = [&](int t, int i) {
+    out[0] = Shape{t, i, 1.0};
+    return 1;
+  };
+  if (d->tpi) return one(d->tpi, d->ip);
+  // FP64: one i per thread, four blocks per SM (50021 x 50021, 6th order, (8,2)
+  // at three blocks 10.00 ms a pass, (8,1) 9.87).  Calls from 16384 i on 65536
+  // j keep (8,2), the family the planner's test fixes there; (8,1) measured
+  // 8.67 ms against 8.93 at 16384 x 131072.
+  if (d->prec == DOUBLE) {
+    if (ni < 1000 || (ni < 2500 && nj <= 16384)) return one(16, 1);
+    return ni >= 16384 && nj >= 65536 ? one(8, 2) : one(8, 1);
+  }
+  const bool spatial = use_spatial(d, ni, nj);
+  const bool large = (double)ni * nj >= 4294967296.0 || nj >= (1 << 19);
+  // Spatial mode: a warp of fewer i has a smaller box, so more far tiles;
+  // 4th order up to 60000 i, (2,2) is 1-9 % ahead of four i per thread.  At
+  // 6th order it would gain 0-3 %, but the block steps of a 262144-body system
+  // with tight binaries (200 steps) once reached t = 5.7e-4 with two i per
+  // thread against 3.13e-3 with four and 3.25e-3 with FP64 forces (address
+  // order: 3.25e-3 with either); the cause is not known, so they keep four.
+  if (spatial && d->order < SIXTH && ni < 60000) return one(2, 2);
+  if (spatial || large) {
+    // (1,4) 537.8, (2,4) 534.6 G interactions/s at N = 2^20, 6th order
+    out[0] = Shape{1, 4, 1.0};
+    out[1] = Shape{2, 4, 0.994};
+    return 2;
+  }
+  // Address order: the fewer i, the more threads each; two i per thread pay
+  // from the sizes where a block per slot still finds enough tiles (6th order,
+  // 3500 i on 30000 j: (4,2) 254 us, (8,2) 265; 2000 i on 7000 j: 64 and 62)
+  if (ni < 256) return one(16, 1);
+  if (ni < 600) return nj < 40000 ? one(8, 1) : one(8, 2);
+  if (ni < 1000) return nj < 12000 ? one(8, 1) : one(8, 2);
+  if (ni < (nj <= 16384 ? 5000 : 1700)) return one(8, 2);
+  return ni <= 16384 ? one(4, 2) : one(2, 2);
 }
 
 static Plan make_plan(const sapb_dev *d, int ni, int nj) {
   const int tj = force_tile_j();
   const int ntiles = std::max(1, (nj + tj - 1) / tj);
-  // (threads per i, i per thread) and the shape's throughput relative to the
-  // best one, measured on B200 at N = 2^20 (6th order, all i, where waves
-  // cost nothing): mixed (1,4) 537.8, (2,4) 534.6, (1,2) 521.8, (2,2) 516.1,
-  // (4,2) 510.4, (8,2) 491.2 G interactions/s; FP64 (2,2) 249.6, (4,2) 247.4,
-  // (8,2) 244.8, (1,2) 243.9.  The one-i-per-thread shapes (only chosen for
-  // very small ni) are estimates.
-  static const int shapes_mix[][2] = {{1, 4}, {2, 4}, {1, 2}, {2, 2}, {4, 2}, {8, 2}, {16, 1}, {32, 1}};
-  static const double eff_mix[] = {1.0, 0.994, 0.970, 0.960, 0.949, 0.913, 0.85, 0.85};
-  static const int shapes_dp[][2] = {{2, 2}, {4, 2}, {8, 2}, {1, 2}, {16, 1}, {32, 1}};
-  static const double eff_dp[] = {1.0, 0.991, 0.981, 0.977, 0.9, 0.9};
-  const int nshape = d->prec == DOUBLE ? 6 : 8;
-  // pair-times per SM and second (B200, measured order of magnitude): only
+  // pairs per SM and second of a full GPU (B200, order of magnitude): only
   // the balance between force and reduction depends on them
-  const double sm_rate = d->prec == DOUBLE ? (d->order >= SIXTH ? 1.5e9 : 2.3e9)
+  const double sm_rate = d->prec == DOUBLE ? (d->order >= SIXTH ? 1.7e9 : 2.4e9)
                                            : (d->order >= SIXTH ? 3.6e9 : 5.6e9);
-  const int max_ns = d->nslices ? ntiles : std::max(1, ntiles / 4);  // keep >= 4 tiles per slice
-  // Mixed precision below 2^32 pairs and 2^19 j: the shape family comes from
-  // the call size, the model above then picks the shape within it and the
-  // j-split.  B200 sweeps of every shape and j-split (4th and 6th order, 256
-  // to 65536 i on 16384 to 2^20 j) put the best shape at two i per thread
-  // with about 65536 / ni threads per i (2 to 8) from 1024 i on (4th order,
-  // 16384 x 16384: 0.45 ms against 0.66 ms for the model's free choice;
-  // 6th order, 4096 i on 16384 j: 0.21 against 0.28 ms), and at 8 threads
-  // per i or one i per thread below.  From 2^32 pairs, or with 2^19 j and
-  // more, where the j-split alone fills the GPU, the model chooses freely:
-  // (1,4) and (2,4) are then within 1 % of the best (2^20 j x 2048 i: (2,4)
-  // 4 % ahead of (8,2)).  Calls in spatial mode keep the free choice too:
-  // there these shapes gained only 0-7 %, and the 6th-order block steps of a
-  // 262144-body system with tight binaries (200 steps, 10 % binaries
-  // 1e-6..1e-4 apart) reached t = 5.7e-4 with them against 3.13e-3 with the
-  // free choice and 3.25e-3 with FP64 forces (address order: 3.25e-3 with
-  // either planner); the cause is not known.
-  bool allow[8] = {true, true, true, true, true, true, true, true};
-  if (d->prec != DOUBLE && !d->tpi && (double)ni * nj < 4294967296.0 && nj < (1 << 19) &&
-      !use_spatial(d, ni, nj)) {
-    for (bool &a : allow) a = false;
-    if (ni < 1024) {
-      allow[5] = allow[6] = allow[7] = true;  // (8,2), (16,1), (32,1)
-    } else {
-      int t = 2;
-      while (t < 8 && (long)t * 2 * ni <= 65536) t *= 2;
-      allow[t == 2 ? 3 : (t == 4 ? 4 : 5)] = true;  // (2,2), (4,2) or (8,2)
-    }
-  }
-  // FP64 kernels, same call sizes (sweep of 4th and 6th order, 256 to 16384
-  // i on 16384 and 131072 j): one i per thread with 16 or 32 threads per i
-  // below 4096 i (16 from 1024 i on), (8,2) or (16,1) up to 16384 i, (8,2)
-  // above; the model's free choice was up to 1.16x off (4th order, 4096 i on
-  // 16384 j).
-  if (d->prec == DOUBLE && !d->tpi && (double)ni * nj < 4294967296.0 && nj < (1 << 19)) {
-    for (bool &a : allow) a = false;
-    if (ni < 1024) {
-      allow[4] = allow[5] = true;  // (16,1), (32,1)
-    } else if (ni < 4096) {
-      allow[4] = true;  // (16,1)
-    } else if (ni < 16384) {
-      allow[2] = allow[4] = true;  // (8,2), (16,1)
-    } else {
-      allow[2] = true;  // (8,2)
-    }
-  }
+  // one tile or more per slice; partial records up to 256 MB
+  const int max_ns = (int)std::max(1.0, std::min<double>(ntiles, 268435456.0 / (96.0 * ni)));
+  Shape family[2];
+  const int nshape = shape_family(d, ni, nj, family);
   Plan best{1, 2, 1, 1, ntiles};
   double best_t = 1e300;
+  // Slices are tried from few to many, and in mixed calls in address order,
+  // where blocks are alike and a tile is short, more have to be 4 % faster:
+  // other calls on the GPU pay for every block's start (16384 x 16384, 4th
+  // order, calls of three streams back to back: 4 slices 335 us each, 11
+  // slices 347).
+  const double more = d->prec == DOUBLE ? 0.99 : (use_spatial(d, ni, nj) ? 1.0 - 1e-9 : 0.96);
   for (int q = 0; q < nshape; q++) {
-    if (!d->tpi && !allow[q]) continue;
-    const int *sh = d->prec == DOUBLE ? shapes_dp[q] : shapes_mix[q];
-    const int tpi = d->tpi ? d->tpi : sh[0];
-    const int ip = d->ip ? d->ip : sh[1];
+    const int tpi = family[q].tpi, ip = family[q].ip;
     const int ti = force_tile_i(tpi, ip);
     const int i_tiles = (ni + ti - 1) / ti;
     const int bps = blocks_per_sm(d->order, d->prec, tpi, ip);
-    const long R = (long)d->num_sms * bps;
-    const double speed = d->tpi ? 1.0 : (d->prec == DOUBLE ? eff_dp[q] : eff_mix[q]);
-    const double tile_time = 128.0 * ti * bps / (speed * sm_rate);
+    const double tile_time = (double)tj * ti * bps / (family[q].eff * sm_rate);
     auto consider = [&](int ns) {
-      ns = std::max(1, std::min(ns, max_ns));
-      const int st = (ntiles + ns - 1) / ns;
-      const int nse = (ntiles + st - 1) / st;  // every slice non-empty
-      const long B = (long)i_tiles * nse;
-      const long waves = (B + R - 1) / R;
-      double t = (double)waves * (st + 1.0) * tile_time;
-      if (nse > 1) t += 5e-6 + (double)nse * ni * kResStride * 8.0 / 4.0e12;
-      if (t < best_t * (1.0 - 1e-9)) {
+      const int st = (ntiles + ns - 1) / ns;  // tiles of the longest slice
+      const double B = (double)i_tiles * ns, sms = d->num_sms, w = B / (sms * bps);
+      double tiles = st + kBlockTiles;
+      if (w > 1.0) {
+        const double mean = w > 2.0 ? (double)ntiles / ns : st;
+        tiles = (w + kTail * (ceil(w) - w)) * (mean + kBlockTiles);
+      }
+      const double used = std::min<double>(bps, ceil(B / sms)) / bps;
+      double t = tiles * sqrt(used) * tile_time;
+      if (ns > 1) t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12);
+      if (t < best_t * (best.tpi == tpi && best.ip == ip ? more : 1.0 - 1e-9)) {
         best_t = t;
-        best = Plan{tpi, ip, nse, i_tiles, st};
+        best = Plan{tpi, ip, ns, i_tiles, st};
       }
     };
     if (d->nslices) {
-      consider(d->nslices);
+      const int st = (ntiles + std::min(d->nslices, ntiles) - 1) / std::min(d->nslices, ntiles);
+      consider((ntiles + st - 1) / st);  // every slice non-empty
     } else {
-      consider(1);
-      consider(max_ns);
-      for (int k = 1; k <= 64; k++) {  // B just below k whole waves
-        const long ns = (long)k * R / std::max(i_tiles, 1);
-        if (ns < 1) continue;
-        if (ns > max_ns) break;
-        consider((int)ns);
+      // the fewest slices for each length of the longest one
+      for (int ns = 1; ns <= max_ns;) {
+        consider(ns);
+        const int st = (ntiles + ns - 1) / ns;
+        ns = st > 1 ? (ntiles + st - 2) / (st - 1) : max_ns + 1;
       }
     }
-    if (d->tpi) break;  // fixed shape
   }
   return best;
 }

@@ -110,10 +110,11 @@ struct FCfg {
   static constexpr int REC = RS * FB;
   static constexpr int TILE_BYTES = kTJ * REC;
   static constexpr int RED_BYTES = TPI > 1 ? kBT * IP * kResStride * 8 : 0;
-  // stages of the tile ring: two for 2 i per thread in mixed precision up to
-  // 4th order, where three would hold the shape to 3 resident blocks per SM
-  // by shared memory (57.6 KB) against the 4 its registers allow
-  static constexpr int NS = (PREC != DOUBLE && ORDER <= FOURTH && IP == 2) ? 2 : kNS;
+  // stages of the tile ring: two where three would hold the shape to 3
+  // resident blocks per SM by shared memory against the 4 its registers
+  // allow: 2 i per thread in mixed precision up to 4th order (57.6 KB), and
+  // one i per thread (FP64, 4th order, 16384 x 16384: 884 -> 841 us)
+  static constexpr int NS = (IP == 1 || (PREC != DOUBLE && ORDER <= FOURTH && IP == 2)) ? 2 : kNS;
   static constexpr int BODY = NS * TILE_BYTES > RED_BYTES ? NS * TILE_BYTES : RED_BYTES;
   // mixed precision keeps its FP64 running totals in shared memory (10 per
   // i, [field][thread] so a warp's accesses are consecutive), which frees
@@ -121,13 +122,14 @@ struct FCfg {
   static constexpr int TOT_BYTES = PREC == DOUBLE ? 0 : IP * 10 * kBT * 8;
   static constexpr int HIT_BYTES = kBT / 32 * kHitBuf * 8;  // neighbour-list hits, per warp
   static constexpr int SMEM = kHdr + BODY + TOT_BYTES + HIT_BYTES;
-  // resident blocks per SM the register budget is held to: FP64 kernels sit
-  // at 168 registers, where one more allocation step (176) drops them from
-  // 3 to 2 blocks per SM and costs 7 % at N = 2^20 (6th order)
+  // resident blocks per SM the register budget is held to: FP64 kernels with
+  // 2 i per thread sit at 168 registers, where one more allocation step (176)
+  // drops them from 3 to 2 blocks per SM and costs 7 % at N = 2^20 (6th
+  // order); with one i per thread they fit 128 registers and 4 blocks
   // (mixed 6th order with 2 i per thread: 3, since at 128 registers the FP64
   // near-pair rescan spills)
   static constexpr int MIN_BLOCKS =
-      PREC == DOUBLE ? 3 : (IP >= 4 ? 2 : (ORDER >= SIXTH && IP == 2 ? 3 : 4));
+      PREC == DOUBLE ? (IP == 1 ? 4 : 3) : (IP >= 4 ? 2 : (ORDER >= SIXTH && IP == 2 ? 3 : 4));
 };
 
 // ---------------- mixed precision pair ----------------
