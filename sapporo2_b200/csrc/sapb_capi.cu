@@ -19,6 +19,18 @@ using namespace sapb;
 
 static char g_err[512];
 
+// Pushes of up to this many j records are copied to a pinned buffer of their
+// own, which the scatter kernel reads over the bus: the caller's staging is
+// free when the call returns, without a copy to the device and a wait for it.  Larger
+// ones are copied and waited for: their copy takes longer than the wait.
+constexpr int kSmallPush = 512;
+// Host force calls of up to this many i read their records from pinned memory
+// inside the predictor's launch and write their results to pinned memory from
+// the reduction; larger ones use the copy engines, which run beside kernels.
+// Both together: 48 j pushed, 48 i on 16384 j through the class 103 -> 87 us;
+// 2001 and 2001 on 100003, 708 -> 692.
+constexpr int kDirectCall = 16384;
+
 // Default accuracy bound of the single-float position difference on far
 // tiles (relative to the pair distance).
 constexpr double kSpatialDelta = 1e-6;
@@ -428,8 +440,14 @@ int sapb_open(sapb_dev **out, int device, int order, int precision, int n_pipes,
     }
     if (cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking) != cudaSuccess) { rc = fail(d, SAPB_ECUDA, "stream"); break; }
     d->stream = d->own_stream;
-    if (cudaEventCreateWithFlags(&d->done, cudaEventDisableTiming) != cudaSuccess) { rc = fail(d, SAPB_ECUDA, "event"); break; }
+    if (cudaEventCreateWithFlags(&d->done, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&d->pushed, cudaEventDisableTiming) != cudaSuccess) {
+      rc = fail(d, SAPB_ECUDA, "event");
+      break;
+    }
     if (cudaMalloc(&d->status_d, sizeof(int)) != cudaSuccess ||
+        cudaHostAlloc(&d->push_h, sizeof(double) * stage_stride(order) * kSmallPush,
+                      cudaHostAllocDefault) != cudaSuccess ||
         cudaHostAlloc(&d->status_h, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
       rc = fail(d, SAPB_ENOMEM, "status word");
       break;
@@ -471,7 +489,9 @@ int sapb_close(sapb_dev *d) {
   if (d->part_d) cudaFree(d->part_d);
   if (d->status_d) cudaFree(d->status_d);
   if (d->status_h) cudaFreeHost(d->status_h);
+  if (d->push_h) cudaFreeHost(d->push_h);
   if (d->done) cudaEventDestroy(d->done);
+  if (d->pushed) cudaEventDestroy(d->pushed);
   if (d->own_stream) cudaStreamDestroy(d->own_stream);
   delete d;
   return SAPB_OK;
@@ -547,6 +567,16 @@ int sapb_push_j(sapb_dev *d, int n) {
     int rc = grow_j(d, std::max(maxaddr + 1, (int)(d->cap * 1.1) + 1));
     if (rc) return rc;
   }
+  if (n <= kSmallPush) {
+    if (d->push_busy) CK(d, cudaEventSynchronize(d->pushed));
+    memcpy(d->push_h, d->stage_h, sizeof(double) * ss * (size_t)n);
+    CK(d, launch_scatter(d->order, d->prec, d->push_h, n, d->cap, d->js, d->pred, d->status_d,
+                         d->stream));
+    d->pred_gen++;
+    CK(d, cudaEventRecord(d->pushed, d->stream));
+    d->push_busy = true;
+    return SAPB_OK;
+  }
   CK(d, cudaMemcpyAsync(d->stage_d, d->stage_h, sizeof(double) * ss * (size_t)n,
                         cudaMemcpyHostToDevice, d->stream));
   CK(d, launch_scatter(d->order, d->prec, d->stage_d, n, d->cap, d->js, d->pred, d->status_d,
@@ -560,7 +590,7 @@ int sapb_push_j(sapb_dev *d, int n) {
 int sapb_predict(sapb_dev *d, int nj, double ti) {
   if (!d || nj < 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "predict of %d j (capacity %d)", nj, d ? d->cap : 0);
   CK(d, cudaSetDevice(d->device));
-  CK(d, launch_predict(d->order, d->prec, nj, ti, d->js, d->pred, d->stream));
+  CK(d, launch_predict(d->order, d->prec, nj, ti, d->js, d->pred, CallPrep{}, d->stream));
   d->pred_gen++;
   return SAPB_OK;
 }
@@ -608,12 +638,14 @@ static float near_r2(const sapb_dev *d, double eps2) {
 // warp's neighbours into a few tiles (8192 i on 131072 j 2.21 against 2.15).
 constexpr int kListBitsMaxJ = 65536;
 
+// `out`: where the results go, res_dev or pinned host memory (`direct`: and the
+// error word to status_h; the list counts are clear already).
 static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double eps2, int flags,
-                     double *res_dev, int *cnt_dev, int *list_dev) {
+                     double *res_dev, int *cnt_dev, int *list_dev, double *out, bool direct) {
   if (nj <= 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
   const Plan P = make_plan(d, ni, nj);
   const bool list = (flags & SAPB_F_NGB_LIST) != 0;
-  if (list) CK(d, cudaMemsetAsync(cnt_dev, 0, sizeof(int) * (size_t)ni, d->stream));
+  if (list && !direct) CK(d, cudaMemsetAsync(cnt_dev, 0, sizeof(int) * (size_t)ni, d->stream));
   ForceArgs A{};
   A.pred = d->pred;
   bool spatial = use_spatial(d, ni, nj);
@@ -650,7 +682,8 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
     A.out = res_dev;
   }
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
-  const ReduceArgs R{A.out, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, A.iperm};
+  const ReduceArgs R{A.out, P.ns, ni, out, A.pred, nj, P.tpi, i_dev, A.iperm, d->status_d,
+                     direct ? d->status_h : nullptr};
   CK(d, launch_reduce(d->order, d->prec, R, d->num_sms, d->stream));
   return SAPB_OK;
 }
@@ -659,20 +692,38 @@ int sapb_force(sapb_dev *d, int nj, int ni, double eps2, double ti, int flags) {
   if (!d) return fail(nullptr, SAPB_EINVAL, "null device");
   if (ni < 0 || ni > d->i_cap) return fail(d, SAPB_EINVAL, "ni = %d (staged capacity %d)", ni, d->i_cap);
   CK(d, cudaSetDevice(d->device));
-  if (flags & SAPB_F_PREDICT) {
-    int rc = sapb_predict(d, nj, ti);
+  const bool predict = (flags & SAPB_F_PREDICT) != 0;
+  const int words = i_stride(d->order) * ni;
+  if (ni == 0 || ni > kDirectCall) {
+    if (predict) {
+      int rc = sapb_predict(d, nj, ti);
+      if (rc) return rc;
+    }
+    d->last_ni = ni;
+    if (ni == 0) return SAPB_OK;
+    CK(d, cudaMemcpyAsync(d->irec_d, d->irec_h, sizeof(double) * (size_t)words,
+                          cudaMemcpyHostToDevice, d->stream));
+    int rc = run_force(d, nj, ni, d->irec_d, eps2, flags, d->res_d, d->ngb_count_d, d->ngb_list_d,
+                       d->res_d, false);
+    if (rc) return rc;
+    CK(d, cudaMemcpyAsync(d->res_h, d->res_d, sizeof(double) * kResStride * (size_t)ni,
+                          cudaMemcpyDeviceToHost, d->stream));
+    CK(d, cudaMemcpyAsync(d->status_h, d->status_d, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
+  } else {
+    if (nj < 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
+    d->last_ni = ni;
+    CallPrep prep;
+    prep.src = d->irec_h;
+    prep.dst = d->irec_d;
+    prep.words = words;
+    prep.ni = ni;
+    if (flags & SAPB_F_NGB_LIST) prep.count = d->ngb_count_d;
+    CK(d, launch_predict(d->order, d->prec, predict ? nj : 0, ti, d->js, d->pred, prep, d->stream));
+    if (predict) d->pred_gen++;
+    int rc = run_force(d, nj, ni, d->irec_d, eps2, flags, d->res_d, d->ngb_count_d, d->ngb_list_d,
+                       d->res_h, true);
     if (rc) return rc;
   }
-  d->last_ni = ni;
-  if (ni == 0) return SAPB_OK;
-  const int is = i_stride(d->order);
-  CK(d, cudaMemcpyAsync(d->irec_d, d->irec_h, sizeof(double) * is * (size_t)ni,
-                        cudaMemcpyHostToDevice, d->stream));
-  int rc = run_force(d, nj, ni, d->irec_d, eps2, flags, d->res_d, d->ngb_count_d, d->ngb_list_d);
-  if (rc) return rc;
-  CK(d, cudaMemcpyAsync(d->res_h, d->res_d, sizeof(double) * kResStride * (size_t)ni,
-                        cudaMemcpyDeviceToHost, d->stream));
-  CK(d, cudaMemcpyAsync(d->status_h, d->status_d, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
   CK(d, cudaEventRecord(d->done, d->stream));
   d->pending = true;
   return SAPB_OK;
@@ -718,7 +769,8 @@ int sapb_force_device(sapb_dev *d, int nj, int ni, const double *i_dev, double e
     return fail(d, SAPB_EINVAL, "neighbour lists requested without buffers");
   CK(d, cudaSetDevice(d->device));
   if (ni == 0) return SAPB_OK;
-  return run_force(d, nj, ni, i_dev, eps2, flags, res_dev, ngb_count_dev, ngb_list_dev);
+  return run_force(d, nj, ni, i_dev, eps2, flags, res_dev, ngb_count_dev, ngb_list_dev, res_dev,
+                   false);
 }
 
 int sapb_wait_selftest(sapb_dev *d, int limit_ms) {
@@ -782,7 +834,8 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
   A.status = d->status_d;
   A.out = scratch;  // every (slice, valid i) record is written before it is read
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
-  const ReduceArgs R{scratch, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, nullptr};
+  const ReduceArgs R{scratch, P.ns, ni, res_dev, A.pred, nj, P.tpi, i_dev, nullptr, nullptr,
+                     nullptr};
   CK(d, launch_reduce(d->order, d->prec, R, d->num_sms, d->stream));
   return SAPB_OK;
 }

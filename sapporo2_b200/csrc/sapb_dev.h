@@ -50,6 +50,10 @@ struct sapb_dev {
   double *stage_h = nullptr;
   double *stage_d = nullptr;
   int stage_cap = 0;
+  // small pushes: a pinned copy the scatter kernel reads, and its last use
+  double *push_h = nullptr;
+  cudaEvent_t pushed = nullptr;
+  bool push_busy = false;
 
   // i records, results
   double *irec_h = nullptr, *irec_d = nullptr;

@@ -139,6 +139,19 @@ struct ReduceArgs {
   int nj, tpi;
   const double *irec;
   const int *iperm;
+  // calls whose `out` is pinned host memory: the device error word is copied
+  // there too (nullptr: not)
+  const int *status;
+  int *status_out;
+};
+
+// What the predictor's launch does for a force call from the host.
+struct CallPrep {
+  const double *src = nullptr;  // i records, pinned host memory
+  double *dst = nullptr;
+  int words = 0;                // doubles to copy
+  int *count = nullptr;         // list counts to clear
+  int ni = 0;
 };
 
 }  // namespace sapb

@@ -16,13 +16,29 @@ namespace sapb {
 // for (reference: dev_copy_particles seeds Ppos/Pvel/Pacc,
 // kernels.cu:281-297).
 // ========================================================================
+// The records of a block (64, 8 to 11 KB) are read whole, in order, into shared
+// memory: a thread reading its own record touches a 128- or 176-byte stride.
+// `stage` may be pinned host memory (small pushes), where that matters most:
+// every read is a bus transaction.
+constexpr int kScatter = 64;
 template <int ORDER, int PREC>
-__global__ void __launch_bounds__(256) scatter_kernel(const double *__restrict__ stage, int n,
-                                                      int cap, JState js, void *pred,
-                                                      int *status) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kScatter) scatter_kernel(const double *__restrict__ stage, int n,
+                                                           int cap, JState js, void *pred,
+                                                           int *status) {
+  constexpr int SS = stage_stride(ORDER);
+  __shared__ __align__(16) double buf[kScatter * (SS + 1)];  // odd stride: no bank conflicts
+  const int first = blockIdx.x * kScatter;
+  const int words = min(kScatter, n - first) * SS;
+  const double *src = stage + (size_t)first * SS;
+#pragma unroll
+  for (int q = 0; q < SS; q++) {
+    const int w = threadIdx.x + q * kScatter;
+    if (w < words) buf[w + w / SS] = src[w];
+  }
+  __syncthreads();
+  const int k = first + threadIdx.x;
   if (k >= n) return;
-  const double *r = stage + (size_t)k * stage_stride(ORDER);
+  const double *r = buf + threadIdx.x * (SS + 1);
   const int addr = __double2loint(r[0]);
   const int id = __double2hiint(r[0]);
   if (addr < 0 || addr >= cap) {
@@ -55,10 +71,22 @@ __global__ void __launch_bounds__(256) scatter_kernel(const double *__restrict__
 // per component and writes the force record of each j.
 // ========================================================================
 // The grid is one wave of resident blocks striding over the j (a grid of
-// nj / 256 blocks would leave its last wave part-empty: 2^20 j are 3.5 waves).
+// nj / 256 blocks would leave its last wave part-empty: 2^20 j are 3.5 waves),
+// then the blocks that prepare a host call: they copy its i records from
+// pinned memory and clear the list counts, beside the predictor and in its
+// launch, instead of a copy and a memset in the stream before it.
 template <int ORDER, int PREC>
-__global__ void __launch_bounds__(256) predict_kernel(int nj, double ti, JState js, void *pred) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nj; k += gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256) predict_kernel(int nj, double ti, JState js, void *pred,
+                                                      int jblocks, CallPrep P) {
+  if ((int)blockIdx.x >= jblocks) {
+    const int w0 = ((int)blockIdx.x - jblocks) * blockDim.x + threadIdx.x;
+    const int step = ((int)gridDim.x - jblocks) * blockDim.x;
+    for (int w = w0; w < P.words; w += step) P.dst[w] = P.src[w];
+    if (P.count)
+      for (int i = w0; i < P.ni; i += step) P.count[i] = 0;
+    return;
+  }
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nj; k += jblocks * blockDim.x) {
     double p[3], v[3], a[3];
     taylor<ORDER>(js, k, ti, p, v, a);
     store_record<ORDER, PREC>(pred, k, p[0], p[1], p[2], __ldg(js.m + k), __ldg(js.id + k),
@@ -613,6 +641,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(ReduceArgs R) {
   int i = valid ? g : 0;
   if (valid && R.iperm) i = __ldg(R.iperm + g);  // spatial mode: neighbours scan the same tiles
   const unsigned char *pred = reinterpret_cast<const unsigned char *>(R.pred);
+  if (R.status_out && blockIdx.x == 0 && threadIdx.x == 0) *R.status_out = *R.status;
   reduce_one<ORDER, PREC, LPI>(
       valid, R.part + (size_t)i * kResStride, (size_t)R.ni * kResStride, R.nslices, R.tpi,
       threadIdx.x & 31, R.irec + (size_t)i * i_stride(ORDER), R.out + (size_t)i * kResStride,
@@ -627,7 +656,8 @@ template <int ORDER, int PREC>
 static cudaError_t launch_scatter_t(const double *stage, int n, int cap, const JState &js,
                                    void *pred, int *status, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  scatter_kernel<ORDER, PREC><<<(n + 255) / 256, 256, 0, st>>>(stage, n, cap, js, pred, status);
+  scatter_kernel<ORDER, PREC>
+      <<<(n + kScatter - 1) / kScatter, kScatter, 0, st>>>(stage, n, cap, js, pred, status);
   return cudaGetLastError();
 }
 
@@ -647,8 +677,7 @@ cudaError_t launch_scatter(int order, int prec, const double *stage, int n, int 
 
 template <int ORDER, int PREC>
 static cudaError_t launch_predict_t(int nj, double ti, const JState &js, void *pred,
-                                    cudaStream_t st) {
-  if (nj <= 0) return cudaSuccess;
+                                    const CallPrep &P, cudaStream_t st) {
   static int wave = 0;  // resident blocks on the whole device (one per instantiation)
   if (!wave) {
     int dev = 0, sms = 0, occ = 0;
@@ -659,22 +688,24 @@ static cudaError_t launch_predict_t(int nj, double ti, const JState &js, void *p
     if (e != cudaSuccess) return e;
     wave = std::max(1, sms * occ);
   }
-  const int blocks = std::min((nj + 255) / 256, wave);
-  predict_kernel<ORDER, PREC><<<blocks, 256, 0, st>>>(nj, ti, js, pred);
+  const int jblocks = std::min((std::max(nj, 0) + 255) / 256, wave);
+  const int blocks = jblocks + (std::max(P.words, P.count ? P.ni : 0) + 1023) / 1024;
+  if (blocks == 0) return cudaSuccess;
+  predict_kernel<ORDER, PREC><<<blocks, 256, 0, st>>>(nj, ti, js, pred, jblocks, P);
   return cudaGetLastError();
 }
 
 cudaError_t launch_predict(int order, int prec, int nj, double ti, const JState &js, void *pred,
-                           cudaStream_t st) {
+                           const CallPrep &P, cudaStream_t st) {
   if (order == GRAPE5) order = FOURTH;  // GRAPE-5 keeps the 4th-order layout
   if (order == FOURTH && prec == DOUBLESINGLE)
-    return launch_predict_t<FOURTH, DOUBLESINGLE>(nj, ti, js, pred, st);
+    return launch_predict_t<FOURTH, DOUBLESINGLE>(nj, ti, js, pred, P, st);
   if (order == FOURTH && prec == DOUBLE)
-    return launch_predict_t<FOURTH, DOUBLE>(nj, ti, js, pred, st);
+    return launch_predict_t<FOURTH, DOUBLE>(nj, ti, js, pred, P, st);
   if (order == SIXTH && prec == DOUBLESINGLE)
-    return launch_predict_t<SIXTH, DOUBLESINGLE>(nj, ti, js, pred, st);
+    return launch_predict_t<SIXTH, DOUBLESINGLE>(nj, ti, js, pred, P, st);
   if (order == SIXTH && prec == DOUBLE)
-    return launch_predict_t<SIXTH, DOUBLE>(nj, ti, js, pred, st);
+    return launch_predict_t<SIXTH, DOUBLE>(nj, ti, js, pred, P, st);
   return cudaErrorInvalidValue;
 }
 

@@ -6,8 +6,9 @@ namespace sapb {
 
 cudaError_t launch_scatter(int order, int prec, const double *stage, int n, int cap,
                            const JState &js, void *pred, int *status, cudaStream_t st);
+// Predicts j[0, nj) (nj 0: none) and prepares a host call (P, may be empty).
 cudaError_t launch_predict(int order, int prec, int nj, double ti, const JState &js, void *pred,
-                           cudaStream_t st);
+                           const CallPrep &P, cudaStream_t st);
 cudaError_t launch_force(int order, int prec, const ForceArgs &A, int tpi, int ip,
                          cudaStream_t st);
 cudaError_t launch_reduce(int order, int prec, const ReduceArgs &R, int sms, cudaStream_t st);
