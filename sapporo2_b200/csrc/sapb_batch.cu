@@ -4,10 +4,10 @@
 // its own prediction time and softening.  Declared in include/sapporo_b200.h.
 //
 // Per run: one H2D copy of a packed host blob (parameters, cluster table,
-// work items, i records), one CUDA graph launch (queue reset, list-count
-// reset, per-cluster predictor, persistent force kernel, slice reduction;
-// captured once and replayed while the capacities stay the same), one D2H
-// copy of the results.
+// work items, i records) and one CUDA graph launch (queue reset, list-count
+// reset, per-cluster predictor, persistent force kernel, slice reduction,
+// which writes the results and the error word to pinned host memory; captured
+// once and replayed while the capacities stay the same).
 #include <stdio.h>
 #include <string.h>
 
@@ -42,8 +42,14 @@ struct sapb_batch {
   int force_blocks = 0;
   cudaEvent_t done = nullptr;
   bool pending = false;
-  int tpi_scale = 0;     // autotuner: log2 factor applied to the threads-per-i rule
-  int split_factor = 4;  // autotuner: work items per resident block targeted by the j-split
+  // Autotuner's parameters and their defaults: log2 factor applied to the
+  // threads-per-i rule, and work items per resident block targeted by the
+  // j-split.  Smaller i-tiles than the rule's balance better and leave the
+  // reduction shorter rows to scan (B200, one run, factor 1 -> 4: 192 clusters
+  // 1190 -> 1176 us, 103 small ones 132 -> 119, 13 with 719 i 70 -> 55; the
+  // autotuner picks 2 or 4 in these).
+  int tpi_scale = 2;
+  int split_factor = 4;
   int runs = 0;
   // inputs of the last plan (re-planned by the autotuner)
   std::vector<int> p_jf, p_jc, p_ic;
@@ -282,6 +288,8 @@ int sapb_batch_run(sapb_batch *b, int flags) {
     B.items = reinterpret_cast<const BatchItem *>(b->blob_d + b->off_it);
     B.irec = reinterpret_cast<const double *>(b->blob_d + b->off_i);
     B.res = b->res_d;
+    B.out = b->res_h;
+    B.status_out = d->status_h;
     B.part = b->part_d;
     B.ngb_count = b->cnt_d;
     B.ngb_list = b->lst_d;
@@ -316,10 +324,6 @@ int sapb_batch_run(sapb_batch *b, int flags) {
   BK(b, cudaMemcpyAsync(b->blob_d, b->blob_h, used_i, cudaMemcpyHostToDevice, d->stream));
   BK(b, cudaGraphLaunch(b->exec, d->stream));
   if (predict) d->pred_gen++;  // the graph's predictor rewrote the records
-  if (b->total_i > 0)
-    BK(b, cudaMemcpyAsync(b->res_h, b->res_d, sizeof(double) * kResStride * (size_t)b->total_i,
-                          cudaMemcpyDeviceToHost, d->stream));
-  BK(b, cudaMemcpyAsync(d->status_h, d->status_d, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
   BK(b, cudaEventRecord(b->done, d->stream));
   b->pending = true;
   b->runs++;

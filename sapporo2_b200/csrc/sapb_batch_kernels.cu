@@ -315,6 +315,7 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs B) {
   const BatchParams &P = *B.par;
   const int lane = threadIdx.x & 31;
   const unsigned char *pred = reinterpret_cast<const unsigned char *>(B.pred);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *B.status_out = *B.status;
   for (int i0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PW; i0 < P.total_i;
        i0 += (int)((gridDim.x * blockDim.x) >> 5) * PW) {
     const int i = i0 + lane / LPI;
@@ -325,12 +326,13 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchArgs B) {
     const bool valid = c >= 0 && i < CL.i_first + CL.i_count;
     const int S = CL.nslices;
     const int sl = (CL.j_count + S - 1) / S;  // j per slice
-    double *out = B.res + (size_t)(valid ? i : 0) * kResStride;
+    const size_t at = (size_t)(valid ? i : 0) * kResStride;
     reduce_one<ORDER, PREC, LPI>(
         valid,
-        valid && S > 1 ? B.part + ((size_t)CL.part_base + (i - CL.i_first)) * kResStride : out,
+        valid && S > 1 ? B.part + ((size_t)CL.part_base + (i - CL.i_first)) * kResStride
+                       : B.res + at,
         (size_t)CL.i_count * kResStride, S, CL.tpi, lane,
-        B.irec + (size_t)(valid ? i : 0) * i_stride(ORDER), out,
+        B.irec + (size_t)(valid ? i : 0) * i_stride(ORDER), B.out + at,
         [&](int s, unsigned t) { return pred + (size_t)(CL.j_first + s * sl + (int)t * kTJ) * REC; },
         [&](int s, unsigned t) {
           return min(kTJ, min(sl, CL.j_count - s * sl) - (int)t * kTJ);

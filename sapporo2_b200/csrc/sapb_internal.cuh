@@ -120,7 +120,9 @@ struct BatchArgs {
   const BatchItem *items;
   BatchParams *par;
   const double *irec;
-  double *res;
+  double *res;        // one record per i; unsplit clusters' before the reduction
+  double *out;        // results, pinned host memory
+  int *status_out;    // the error word, too
   double *part;
   int *ngb_count, *ngb_list;
   int do_list, do_predict;

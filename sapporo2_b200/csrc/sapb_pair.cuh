@@ -830,8 +830,14 @@ __device__ __forceinline__ void reduce_one(bool valid, const double *part, size_
       ax = (double)__uint_as_float((unsigned)(key >> 32));
       ay = (double)(int)(unsigned)key;
     }
-    out[2 * l] = ax;
-    out[2 * l + 1] = ay;
+    // whole 16-byte words where the caller's pointer allows it: `out` may be
+    // pinned host memory, each store a bus transaction
+    if ((reinterpret_cast<size_t>(out) & 15) == 0) {
+      reinterpret_cast<double2 *>(out)[l] = make_double2(ax, ay);
+    } else {
+      out[2 * l] = ax;
+      out[2 * l + 1] = ay;
+    }
   }
 }
 
