@@ -439,16 +439,16 @@ __global__ void __launch_bounds__(kT, 2) mlp_backward_kernel(const float *__rest
 // 32 threads for each, striding over the rows: a full grid's 296 rows (10 MB,
 // from L2) are ten loads per thread, all in flight together (with eight
 // threads per parameter it took 10.5 us of the epoch, under ncu).
-// The moments' weights and bias corrections are rounded once, from double: in
-// float, 1 - 0.999f is 1.3e-5 off and 1 - 0.999f^8 4e-6, and every step's
-// length with it.
+// The step is taken in FP64 on the FP32 moments and parameters: with FP32
+// constants 1 - 0.999f is 1.3e-5 off and 1 - 0.999f^8 4e-6, the same for every
+// parameter, and the loss after a few epochs of a steep start moves by ten
+// times as much.
 struct AdamStep {
-  float lr, b1, d1, b2, d2, eps, c1, c2;  // d = 1 - b, c = 1 - b^step
+  double lr, b1, b2, eps, c1, c2;  // c = 1 - b^step
 };
 static AdamStep adam_step(float lr, int step) {
   const double b1 = 0.9, b2 = 0.999;
-  return AdamStep{lr, (float)b1, (float)(1.0 - b1), (float)b2, (float)(1.0 - b2), 1e-8f,
-                  (float)(1.0 - pow(b1, step)), (float)(1.0 - pow(b2, step))};
+  return AdamStep{(double)lr, b1, b2, 1e-8, 1.0 - pow(b1, step), 1.0 - pow(b2, step)};
 }
 __global__ void __launch_bounds__(1024) mlp_update_kernel(const float *__restrict__ part, int rows,
                                                           float *P, float *M, float *V, AdamStep a,
@@ -468,17 +468,17 @@ __global__ void __launch_bounds__(1024) mlp_update_kernel(const float *__restric
 #pragma unroll
   for (int r = 0; r < 32; r++) s += red[r][c];
   if (k > kNP) return;
-  const float g = (float)s;
+  const double g = s;
   if (k == kNP) {
-    *loss = g;
+    *loss = (float)g;
   } else if (M) {
-    const float m = a.b1 * M[k] + a.d1 * g;
-    const float v = a.b2 * V[k] + a.d2 * g * g;
-    M[k] = m;
-    V[k] = v;
-    P[k] -= a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+    const double m = a.b1 * M[k] + (1.0 - a.b1) * g;
+    const double v = a.b2 * V[k] + (1.0 - a.b2) * g * g;
+    M[k] = (float)m;
+    V[k] = (float)v;
+    P[k] = (float)(P[k] - a.lr * (m / a.c1) / (sqrt(v / a.c2) + a.eps));
   } else {
-    G[k] = g;
+    G[k] = (float)g;
   }
 }
 
