@@ -458,6 +458,8 @@ int sapb_open(sapb_dev **out, int device, int order, int precision, int n_pipes,
     if (rc) break;
     rc = ensure_i(d, d->n_pipes);
     if (rc) break;
+    rc = ensure_part(d, 1 << 18);  // 2 MB: the first small calls find their partial sums' room
+    if (rc) break;
     rc = noalloc_setup(d);
     if (rc) break;
     if (cudaStreamSynchronize(d->stream) != cudaSuccess) { rc = fail(d, SAPB_ECUDA, "sync"); break; }
