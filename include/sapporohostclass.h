@@ -66,8 +66,17 @@ class sapporo {
   std::vector<int> stage_slot_;
   std::vector<std::vector<int> > staged_addr_;
 
-  // per-address prediction time of the force records (NaN: unpredicted copy)
+  // prediction time of each address's force record (NaN: unpredicted copy):
+  // that of the last call that predicted the first pred_nj_ addresses, unless
+  // pushed_ says that the address was pushed since (pred_epoch_ counts those
+  // calls); pred_time_ for addresses that the last call did not reach
   std::vector<double> pred_time_;
+  std::vector<unsigned> pushed_;
+  double pred_t_;
+  int pred_nj_;
+  unsigned pred_epoch_;
+  void note_prediction(int nj);
+  double predicted_at(int addr) const;
   std::vector<double> jcache_;   // 24 doubles per address, see sapb_read_j
   int jcache_n_;
 

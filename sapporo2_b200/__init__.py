@@ -44,29 +44,35 @@ LIB_PATH = Path(os.environ.get("SAPPORO_B200_LIB", _PKG / "lib" / "libsapporo_b2
 
 _lib = None
 
-_dp = np.ctypeslib.ndpointer(dtype=np.float64, flags="C_CONTIGUOUS")
-_ip = np.ctypeslib.ndpointer(dtype=np.int32, flags="C_CONTIGUOUS")
-
-
 class SapporoError(RuntimeError):
     pass
 
 
-def _opt(ptr_type):
-    """ndpointer that also accepts None."""
+class _Array:
+    """ctypes argument type for a C-contiguous numpy array (or, `optional`, None).
 
-    class _P(ptr_type):  # type: ignore[misc, valid-type]
-        @classmethod
-        def from_param(cls, obj):
-            if obj is None:
-                return None
-            return ptr_type.from_param(obj)
+    np.ctypeslib.ndpointer checks and passes an array in several microseconds,
+    two dozen times in a block step; the writable array of the right type that
+    the methods below make themselves goes through the buffer protocol instead.
+    Everything else (read-only, empty, wrong type or layout) is ndpointer's."""
 
-    return _P
+    def __init__(self, dtype, optional=False):
+        self.dtype, self.optional = np.dtype(dtype), optional
+        self.general = np.ctypeslib.ndpointer(dtype=dtype, flags="C_CONTIGUOUS")
+
+    def from_param(self, obj):
+        if obj is None and self.optional:
+            return None
+        if type(obj) is np.ndarray and obj.dtype is self.dtype and obj.flags.c_contiguous:
+            try:
+                return C.byref(C.c_char.from_buffer(obj))
+            except (TypeError, ValueError):
+                pass
+        return self.general.from_param(obj)
 
 
-_dpo = _opt(_dp)
-_ipo = _opt(_ip)
+_dp, _ip = _Array(np.float64), _Array(np.int32)
+_dpo, _ipo = _Array(np.float64, optional=True), _Array(np.int32, optional=True)
 
 # (name, restype, argtypes)
 _SIGS = [

@@ -69,8 +69,19 @@ void g5_set_eps2_to_all(double eps2) { eps_to_use = eps2; }
 void g5_set_eps_to_all(double eps) { eps_to_use = eps * eps; }
 
 void g5_set_xmj(int addr, int nj, double xj[][3], double jmass[]) {
+  // one bulk upload; arrays indexed by address (:111-115), ids = addresses
+  if (nj <= 0) return;
+  if (addr >= 0) {
+    std::vector<int> at((size_t)nj);
+    for (int i = 0; i < nj; i++) at[i] = addr + i;
+    if (grav5.set_j_particles(nj, at.data(), at.data(), nullptr, jmass + addr, xj[addr], nullptr,
+                              nullptr, nullptr, nullptr, nullptr, nullptr) == 0)
+      return;
+  }
+  // refused as a whole (an address beyond the j memory): one by one, as far as
+  // they go
   double z[3] = {0, 0, 0};
-  for (int i = addr; i < addr + nj; i++)  // :111-115: arrays indexed by address
+  for (int i = addr; i < addr + nj; i++)
     grav5.set_j_particle(i, i, 0.0, 0.0, jmass[i], z, z, z, z, xj[i], z, z, 0.0);
 }
 

@@ -62,6 +62,9 @@ sapporo::sapporo()
       predict(false),
       nj_updated(false),
       predJOnHost(false),
+      pred_t_(NAN),
+      pred_nj_(0),
+      pred_epoch_(1),
       jcache_n_(0),
       dev_ni(0),
       nj_last_(0),
@@ -111,6 +114,10 @@ int sapporo::open(std::string kernelFile, int *devices, int nprocs, int order, i
   nj_max = 16384;  // lib/src/sapporohostclass.cpp:161-162
   stage_slot_.assign(nj_max, -1);
   pred_time_.assign(nj_max, NAN);
+  pushed_.assign(nj_max, 0u);
+  pred_t_ = NAN;
+  pred_nj_ = 0;
+  pred_epoch_ = 1;
   staged_addr_.assign((size_t)G, std::vector<int>());
   dev_nj_.assign((size_t)G, 0);
   ngb_count_h_.assign((size_t)G, std::vector<int>());
@@ -165,6 +172,7 @@ void sapporo::increase_jMemory() {
   nj_max = temp;
   stage_slot_.resize(nj_max, -1);
   pred_time_.resize(nj_max, NAN);
+  pushed_.resize(nj_max, 0u);
   for (sapb_dev *d : devs_) {
     const int rc = sapb_reserve_j(d, nj_max / G);
     if (rc) report("reserve_j", rc, d);
@@ -369,6 +377,7 @@ int sapporo::push_staged() {
     for (int a : staged) {
       stage_slot_[a] = -1;
       pred_time_[a] = NAN;
+      pushed_[a] = pred_epoch_;
     }
     staged.clear();
     if (r) {
@@ -378,6 +387,23 @@ int sapporo::push_staged() {
   }
   nj_updated = false;
   return rc;
+}
+
+// The first nj addresses have been predicted to t_i.  Noted as a whole: one
+// time per address (1 MB at 131072 j) took longer than the launches of a call.
+void sapporo::note_prediction(int nj) {
+  nj = std::min(nj, (int)pred_time_.size());
+  for (int k = std::max(nj, 0); k < pred_nj_; k++)  // reached by the call before only
+    if (pushed_[k] != pred_epoch_) pred_time_[k] = pred_t_;
+  pred_t_ = t_i;
+  pred_nj_ = nj;
+  pred_epoch_++;
+}
+
+double sapporo::predicted_at(int addr) const {
+  if (addr >= (int)pred_time_.size()) return NAN;
+  if (addr < pred_nj_ && pushed_[addr] != pred_epoch_) return pred_t_;
+  return pred_time_[addr];
 }
 
 void sapporo::send_j_particles_to_device() {
@@ -452,7 +478,7 @@ void sapporo::startGravCalc(int nj, int ni, int id[], double xi[][3], double vi[
     }
   }
   if (!rc && predict)
-    for (int k = 0; k < nj && k < (int)pred_time_.size(); k++) pred_time_[k] = t_i;
+    note_prediction(nj);
   last_status = rc;
   dev_ni = ni;
   nj_last_ = nj;
@@ -592,7 +618,7 @@ void sapporo::forcePrediction(int nj) {
     if (rc) report("forcePrediction", rc, devs_[g]);
   }
   if (!rc && predict && nj > 0)
-    for (int k = 0; k < nj && k < (int)pred_time_.size(); k++) pred_time_[k] = t_i;
+    note_prediction(nj);
   last_status = rc;
   predict = false;
 }
@@ -636,7 +662,7 @@ int sapporo::refresh_jcache(int addr) {
     predJOnHost = true;
   }
   if (addr >= jcache_n_) return SAPB_EINVAL;
-  const double pt = addr < (int)pred_time_.size() ? pred_time_[addr] : NAN;
+  const double pt = predicted_at(addr);
   if (std::isnan(pt) || pt != t_i) {
     double one[24];
     const int rc = sapb_read_j(devs_[addr % G], addr / G, 1, std::isnan(pt) ? 0.0 : pt,

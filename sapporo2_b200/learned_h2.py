@@ -60,6 +60,15 @@ def retry_h2(h2, count, target=TARGET) -> np.ndarray:
     return np.asarray(h2) * (target / np.maximum(np.asarray(count, dtype=np.float64), 1.0)) ** (2.0 / 3.0)
 
 
+def _fp(a):
+    """A float32 array as a pointer argument (the buffer protocol where it
+    can; ndarray.ctypes takes several microseconds)."""
+    try:
+        return C.byref(C.c_float.from_buffer(a))
+    except (TypeError, ValueError):  # read-only or empty
+        return a.ctypes.data_as(C.POINTER(C.c_float))
+
+
 class H2Net:
     """The network on the GPU of an open :class:`Sapporo` instance."""
 
@@ -81,7 +90,7 @@ class H2Net:
 
     def params(self) -> np.ndarray:
         p = np.zeros(self.np, dtype=np.float32)
-        _check(self.lib.sapb_mlp_get_params(self.h, p.ctypes.data_as(C.POINTER(C.c_float))),
+        _check(self.lib.sapb_mlp_get_params(self.h, _fp(p)),
                "mlp_get", self.owner.dev)
         return p
 
@@ -95,7 +104,7 @@ class H2Net:
 
     def set_params(self, p):
         p = np.ascontiguousarray(p, dtype=np.float32)
-        _check(self.lib.sapb_mlp_set_params(self.h, p.ctypes.data_as(C.POINTER(C.c_float))),
+        _check(self.lib.sapb_mlp_set_params(self.h, _fp(p)),
                "mlp_set", self.owner.dev)
 
     @staticmethod
@@ -105,8 +114,8 @@ class H2Net:
     def forward(self, x) -> np.ndarray:
         x = self._f(x)
         y = np.zeros(len(x), dtype=np.float32)
-        _check(self.lib.sapb_mlp_forward(self.h, len(x), x.ctypes.data_as(C.POINTER(C.c_float)),
-                                         y.ctypes.data_as(C.POINTER(C.c_float))), "mlp_forward",
+        _check(self.lib.sapb_mlp_forward(self.h, len(x), _fp(x),
+                                         _fp(y)), "mlp_forward",
                self.owner.dev)
         return y
 
@@ -114,17 +123,17 @@ class H2Net:
         x, t = self._f(x), self._f(t)
         g = np.zeros(self.np, dtype=np.float32)
         loss = C.c_float()
-        _check(self.lib.sapb_mlp_gradient(self.h, len(x), x.ctypes.data_as(C.POINTER(C.c_float)),
-                                          t.ctypes.data_as(C.POINTER(C.c_float)),
-                                          g.ctypes.data_as(C.POINTER(C.c_float)), C.byref(loss)),
+        _check(self.lib.sapb_mlp_gradient(self.h, len(x), _fp(x),
+                                          _fp(t),
+                                          _fp(g), C.byref(loss)),
                "mlp_gradient", self.owner.dev)
         return g, loss.value
 
     def train(self, x, t, epochs=20, lr=1e-3) -> float:
         x, t = self._f(x), self._f(t)
         loss = C.c_float()
-        _check(self.lib.sapb_mlp_train(self.h, len(x), x.ctypes.data_as(C.POINTER(C.c_float)),
-                                       t.ctypes.data_as(C.POINTER(C.c_float)), int(epochs),
+        _check(self.lib.sapb_mlp_train(self.h, len(x), _fp(x),
+                                       _fp(t), int(epochs),
                                        float(lr), C.byref(loss)), "mlp_train", self.owner.dev)
         return loss.value
 
@@ -171,11 +180,9 @@ class H2Net:
         mu = self._f(self.mu)
         sd = self._f(self.sd)
         out = np.empty(n, dtype=np.float32)
-        fp = C.POINTER(C.c_float)
-        _check(self.lib.sapb_mlp_propose(self.h, n, rec.ctypes.data_as(fp), mu.ctypes.data_as(fp),
-                                         sd.ctypes.data_as(fp), float(TARGET),
+        _check(self.lib.sapb_mlp_propose(self.h, n, _fp(rec), _fp(mu), _fp(sd), float(TARGET),
                                          float(self.MAX_DOWN), float(self.MAX_UP), float(clip),
-                                         out.ctypes.data_as(fp)), "mlp_propose", self.owner.dev)
+                                         _fp(out)), "mlp_propose", self.owner.dev)
         return out.astype(np.float64)
 
     def propose_host(self, n_prev, h2_prev, acc, jrk, lrho_mean=None, clip=4.0) -> np.ndarray:
