@@ -224,9 +224,8 @@ static int blocks_per_sm(int order, int prec, int tpi, int ip) {
 
 // Launch shape for ni i-particles and nj j.
 //
-// Threads per i and i per thread come from the call's size (shape_family,
-// from sweeps of every shape and j-split on B200); where two are given the
-// cost below decides.  The number of j-slices S minimises the cost of
+// Threads per i and i per thread come from shape_mixed or shape_fp64.  The
+// number of j-slices S minimises the cost of
 // B = i-tiles x S blocks in R = SMs x resident blocks slots: a block costs
 // its tiles plus kBlockTiles for its start and end; up to one wave the call
 // takes as long as its longest block, beyond that as long as the slots take
@@ -234,57 +233,110 @@ static int blocks_per_sm(int order, int prec, int tpi, int ip) {
 // With a share u of an SM's slots in use a tile takes sqrt(u) of its time on
 // a full SM (latency, not the pipe, bounds a block there).  Each slice adds
 // its records to the reduction, and kSliceS to that kernel's chain of loads.
-// Over 130 calls of 4 to 16384 i on 1024 to 131072 j, lists on, the plans are
-// within 2.4 % of the best of the sweep on average; the previous ones (whole
-// waves, a tile for every block's start, four tiles or more per slice, larger
-// shapes) within 8 to 12 %.
 constexpr double kBlockTiles = 0.3, kTail = 0.6, kSliceS = 5e-8;
 extern "C" {
 static bool use_spatial(const sapb_dev *d, int ni, int nj);  // defined with the C ABI below
 }
 
+// Spatial mode pays for its per-call work (the i sort and bounds, the j
+// gather after each prediction) from about 2^28 pairs, 1024 i and 65536 j on
+// (B200, predict + force per call, neighbour lists on, i a random subset of
+// the j: 1.04-1.06 x at 2^28 with 65536 to 262144 j, 1.07-1.12 x from 2^31;
+// 0.89-0.95 x at 2^28 with 16384 or 32768 j, 0.91-1.00 x at 2^26 and 2^27;
+// block-step active sets, which are spatially clustered, gain more);
+// smaller calls run in address order.
+constexpr double kSpatialMinPairs = 268435456.0;  // 2^28
+constexpr int kSpatialMinI = 1024;
+constexpr int kSpatialMinJ = 65536;
+
 struct Shape {
   int tpi, ip;
-  double eff;  // throughput of a full GPU relative to the others of its family
 };
 
-static int shape_family(const sapb_dev *d, int ni, int nj, Shape out[2]) {
-  auto one = [&](int t, int i) {
-    out[0] = Shape{t, i, 1.0};
-    return 1;
-  };
-  if (d->tpi) return one(d->tpi, d->ip);
-  // FP64: one i per thread, four blocks per SM (50021 x 50021, 6th order, (8,2)
-  // at three blocks 10.00 ms a pass, (8,1) 9.87).  Calls from 16384 i on 65536
-  // j keep (8,2), the family the planner's test fixes there; (8,1) measured
-  // 8.67 ms against 8.93 at 16384 x 131072.
-  if (d->prec == DOUBLE) {
-    if (ni < 1000 || (ni < 2500 && nj <= 16384)) return one(16, 1);
-    return ni >= 16384 && nj >= 65536 ? one(8, 2) : one(8, 1);
-  }
+// Mixed precision.  The fewer threads per i, the longer the FP32 sums before
+// they are folded to FP64 (256 / TPI records): the acceleration's relative
+// error, rms against FP64 (4000 i on 262144 j, spatial mode), is 2.5e-8 with
+// (16,1), 3.1e-8 with (8,2), 3.2e-8 with (4,2), 3.6e-8 with (2,4) or (2,2) and
+// 5.1e-8 with (1,4).  Time steps of tight binaries follow that rounding, so a
+// shape gives way to a faster one only where that has as many threads per i.
+// (Families with fewer, (8,1) for (32,1) below 1024 i, (4,2) for (8,2) below
+// 8192, (1,4) or (2,4) for all calls in spatial mode, were 1-30 % faster, with
+// errors up to 1.9 times as large.)
+//
+// Free choice among all shapes, or below 2^32 pairs and 2^19 j in address order
+// among those of the call's size (two i per thread with about 65536 / ni
+// threads per i from 1024 i on: 16384 x 16384, 4th order, 0.45 ms against
+// 0.66 for the free choice; 8 or more threads per i below), by the time of whole
+// waves of blocks of four tiles or more, a tile more for a block's start.
+static Shape shape_mixed(const sapb_dev *d, int ni, int nj) {
+  static const Shape shapes[] = {{1, 4}, {2, 4}, {1, 2}, {2, 2}, {4, 2}, {8, 2}, {16, 1}, {32, 1}};
+  // throughput of a full GPU: 537.8, 534.6, 521.8, 516.1, 510.4 and 491.2 G
+  // interactions/s at N = 2^20, 6th order; the last two are estimates
+  static const double eff[] = {1.0, 0.994, 0.970, 0.960, 0.949, 0.913, 0.85, 0.85};
   const bool spatial = use_spatial(d, ni, nj);
-  const bool large = (double)ni * nj >= 4294967296.0 || nj >= (1 << 19);
-  // Spatial mode: a warp of fewer i has a smaller box, so more far tiles;
-  // 4th order up to 60000 i, (2,2) is 1-9 % ahead of four i per thread.  At
-  // 6th order it would gain 0-3 %, but the block steps of a 262144-body system
-  // with tight binaries (200 steps) once reached t = 5.7e-4 with two i per
-  // thread against 3.13e-3 with four and 3.25e-3 with FP64 forces (address
-  // order: 3.25e-3 with either); the cause is not known, so they keep four.
-  if (spatial && d->order < SIXTH && ni < 60000) return one(2, 2);
-  if (spatial || large) {
-    // (1,4) 537.8, (2,4) 534.6 G interactions/s at N = 2^20, 6th order
-    out[0] = Shape{1, 4, 1.0};
-    out[1] = Shape{2, 4, 0.994};
-    return 2;
+  // spatial mode asked for at any size: few i take the shapes of address order
+  // (6th order, 1 i on 131072 j, host call: 77 us against 156 with (1,4))
+  const bool ordered = spatial && ni >= kSpatialMinI && nj >= kSpatialMinJ;
+  int first = 0, last = 7;
+  if ((double)ni * nj < 4294967296.0 && nj < (1 << 19) && !ordered) {
+    int t = 2;
+    while (t < 8 && (long)t * 2 * ni <= 65536) t *= 2;
+    first = ni < 1024 ? 5 : (t == 2 ? 3 : (t == 4 ? 4 : 5));
+    if (ni >= 1024) last = first;
   }
-  // Address order: the fewer i, the more threads each; two i per thread pay
-  // from the sizes where a block per slot still finds enough tiles (6th order,
-  // 3500 i on 30000 j: (4,2) 254 us, (8,2) 265; 2000 i on 7000 j: 64 and 62)
-  if (ni < 256) return one(16, 1);
-  if (ni < 600) return nj < 40000 ? one(8, 1) : one(8, 2);
-  if (ni < 1000) return nj < 12000 ? one(8, 1) : one(8, 2);
-  if (ni < (nj <= 16384 ? 5000 : 1700)) return one(8, 2);
-  return ni <= 16384 ? one(4, 2) : one(2, 2);
+  const int tj = force_tile_j(), ntiles = std::max(1, (nj + tj - 1) / tj);
+  const int max_ns = std::max(1, ntiles / 4);
+  const double sm_rate = d->order >= SIXTH ? 3.6e9 : 5.6e9;
+  Shape best = shapes[first];
+  double best_t = 1e300;
+  for (int q = first; q <= last; q++) {
+    const int ti = force_tile_i(shapes[q].tpi, shapes[q].ip);
+    const int i_tiles = std::max(1, (ni + ti - 1) / ti);
+    const int bps = blocks_per_sm(d->order, d->prec, shapes[q].tpi, shapes[q].ip);
+    const long slots = (long)d->num_sms * bps;
+    const double tile_time = 128.0 * ti * bps / (eff[q] * sm_rate);
+    auto consider = [&](int ns) {
+      const int st = (ntiles + ns - 1) / ns, used = (ntiles + st - 1) / st;
+      const long waves = ((long)i_tiles * used + slots - 1) / slots;
+      double t = (double)waves * (st + 1.0) * tile_time;
+      if (used > 1) t += 5e-6 + (double)used * ni * kResStride * 8.0 / 4.0e12;
+      if (t < best_t * (1.0 - 1e-9)) {
+        best_t = t;
+        best = shapes[q];
+      }
+    };
+    if (d->nslices) {
+      consider(std::min(d->nslices, max_ns));
+      continue;
+    }
+    consider(1);
+    consider(max_ns);
+    for (int k = 1; k <= 64; k++) {  // just below k whole waves
+      const long ns = k * slots / i_tiles;
+      if (ns > max_ns) break;
+      if (ns >= 1) consider((int)ns);
+    }
+  }
+  // Spatial mode: at least four threads per i below 60000 i.  What matters there
+  // is that a block step's calls round alike: the sums of one tile, all in one
+  // direction, err differently with each shape, and the corrector's third
+  // differences amplify the change.  200 block steps of 262144 bodies with tight
+  // binaries, five seeds, t reached in 1e-3: so 3.13, 3.45, 3.85, 0.09 and 0.02;
+  // by the times above alone 3.13, 0.02, 3.57, 0.09 and 0.02; (2,4) throughout
+  // 0.24, 3.27, 3.57, 0.21 and 0.02.  (4,2) is 0-3 % slower there than the
+  // fastest shape.  With (2,4) for (1,4) above, the fourth seed reaches 3.66, but
+  // 500009 x 500009 at 6th order takes 413.6 ms instead of 399.6.
+  if (ordered && ni < 60000 && best.tpi < 4) return {4, 2};
+  return best;
+}
+
+// FP64: one i per thread, four blocks per SM (50021 x 50021, 6th order, (8,2)
+// at three blocks 10.00 ms a pass, (8,1) 9.87).  Calls from 16384 i on 65536 j
+// keep (8,2), the family the planner's test fixes there; (8,1) measured 8.67 ms
+// against 8.93 at 16384 x 131072.
+static Shape shape_fp64(int ni, int nj) {
+  if (ni < 1000 || (ni < 2500 && nj <= 16384)) return {16, 1};
+  return ni >= 16384 && nj >= 65536 ? Shape{8, 2} : Shape{8, 1};
 }
 
 static Plan make_plan(const sapb_dev *d, int ni, int nj) {
@@ -296,8 +348,6 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj) {
                                            : (d->order >= SIXTH ? 3.6e9 : 5.6e9);
   // one tile or more per slice; partial records up to 256 MB
   const int max_ns = (int)std::max(1.0, std::min<double>(ntiles, 268435456.0 / (96.0 * ni)));
-  Shape family[2];
-  const int nshape = shape_family(d, ni, nj, family);
   Plan best{1, 2, 1, 1, ntiles};
   double best_t = 1e300;
   // Slices are tried from few to many, and in mixed calls in address order,
@@ -306,38 +356,38 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj) {
   // order, calls of three streams back to back: 4 slices 335 us each, 11
   // slices 347).
   const double more = d->prec == DOUBLE ? 0.99 : (use_spatial(d, ni, nj) ? 1.0 - 1e-9 : 0.96);
-  for (int q = 0; q < nshape; q++) {
-    const int tpi = family[q].tpi, ip = family[q].ip;
-    const int ti = force_tile_i(tpi, ip);
-    const int i_tiles = (ni + ti - 1) / ti;
-    const int bps = blocks_per_sm(d->order, d->prec, tpi, ip);
-    const double tile_time = (double)tj * ti * bps / (family[q].eff * sm_rate);
-    auto consider = [&](int ns) {
-      const int st = (ntiles + ns - 1) / ns;  // tiles of the longest slice
-      const double B = (double)i_tiles * ns, sms = d->num_sms, w = B / (sms * bps);
-      double tiles = st + kBlockTiles;
-      if (w > 1.0) {
-        const double mean = w > 2.0 ? (double)ntiles / ns : st;
-        tiles = (w + kTail * (ceil(w) - w)) * (mean + kBlockTiles);
-      }
-      const double used = std::min<double>(bps, ceil(B / sms)) / bps;
-      double t = tiles * sqrt(used) * tile_time;
-      if (ns > 1) t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12);
-      if (t < best_t * (best.tpi == tpi && best.ip == ip ? more : 1.0 - 1e-9)) {
-        best_t = t;
-        best = Plan{tpi, ip, ns, i_tiles, st};
-      }
-    };
-    if (d->nslices) {
-      const int st = (ntiles + std::min(d->nslices, ntiles) - 1) / std::min(d->nslices, ntiles);
-      consider((ntiles + st - 1) / st);  // every slice non-empty
-    } else {
-      // the fewest slices for each length of the longest one
-      for (int ns = 1; ns <= max_ns;) {
-        consider(ns);
-        const int st = (ntiles + ns - 1) / ns;
-        ns = st > 1 ? (ntiles + st - 2) / (st - 1) : max_ns + 1;
-      }
+  const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
+                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj);
+  const int tpi = sh.tpi, ip = sh.ip;
+  const int ti = force_tile_i(tpi, ip);
+  const int i_tiles = (ni + ti - 1) / ti;
+  const int bps = blocks_per_sm(d->order, d->prec, tpi, ip);
+  const double tile_time = (double)tj * ti * bps / sm_rate;
+  auto consider = [&](int ns) {
+    const int st = (ntiles + ns - 1) / ns;  // tiles of the longest slice
+    const double B = (double)i_tiles * ns, sms = d->num_sms, w = B / (sms * bps);
+    double tiles = st + kBlockTiles;
+    if (w > 1.0) {
+      const double mean = w > 2.0 ? (double)ntiles / ns : st;
+      tiles = (w + kTail * (ceil(w) - w)) * (mean + kBlockTiles);
+    }
+    const double used = std::min<double>(bps, ceil(B / sms)) / bps;
+    double t = tiles * sqrt(used) * tile_time;
+    if (ns > 1) t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12);
+    if (t < best_t * (best_t < 1e299 ? more : 1.0)) {
+      best_t = t;
+      best = Plan{tpi, ip, ns, i_tiles, st};
+    }
+  };
+  if (d->nslices) {
+    const int st = (ntiles + std::min(d->nslices, ntiles) - 1) / std::min(d->nslices, ntiles);
+    consider((ntiles + st - 1) / st);  // every slice non-empty
+  } else {
+    // the fewest slices for each length of the longest one
+    for (int ns = 1; ns <= max_ns;) {
+      consider(ns);
+      const int st = (ntiles + ns - 1) / ns;
+      ns = st > 1 ? (ntiles + st - 2) / (st - 1) : max_ns + 1;
     }
   }
   return best;
@@ -607,17 +657,6 @@ double *sapb_i_stage(sapb_dev *d, int ni) {
   return d->irec_h;
 }
 
-// Spatial mode pays for its per-call work (the i sort and bounds, the j
-// gather after each prediction) from about 2^28 pairs, 1024 i and 65536 j on
-// (B200, predict + force per call, neighbour lists on, i a random subset of
-// the j: 1.04-1.06 x at 2^28 with 65536 to 262144 j, 1.07-1.12 x from 2^31;
-// 0.89-0.95 x at 2^28 with 16384 or 32768 j, 0.91-1.00 x at 2^26 and 2^27;
-// block-step active sets, which are spatially clustered, gain more);
-// smaller calls run in address order.
-constexpr double kSpatialMinPairs = 268435456.0;  // 2^28
-constexpr int kSpatialMinI = 1024;
-constexpr int kSpatialMinJ = 65536;
-
 static bool use_spatial(const sapb_dev *d, int ni, int nj) {
   if (d->prec != DOUBLESINGLE || d->sp.mode == 0) return false;
   if (d->sp.mode == 2) return true;
@@ -645,7 +684,14 @@ constexpr int kListBitsMaxJ = 65536;
 static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double eps2, int flags,
                      double *res_dev, int *cnt_dev, int *list_dev, double *out, bool direct) {
   if (nj <= 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
-  const Plan P = make_plan(d, ni, nj);
+  Plan P = make_plan(d, ni, nj);
+  if (P.ns > 1) {
+    const int rc = ensure_part(d, (size_t)P.ns * ni * kResStride);
+    // no room for the partial sums of a planned split: one slice needs none
+    // (a split that the caller fixed is refused)
+    if (rc && (rc != SAPB_ENOMEM || d->nslices)) return rc;
+    if (rc) P.ns = 1;
+  }
   const bool list = (flags & SAPB_F_NGB_LIST) != 0;
   if (list && !direct) CK(d, cudaMemsetAsync(cnt_dev, 0, sizeof(int) * (size_t)ni, d->stream));
   ForceArgs A{};
@@ -676,13 +722,7 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
   A.ngb_count = cnt_dev;
   A.ngb_list = list_dev;
   A.status = d->status_d;
-  if (P.ns > 1) {
-    int rc = ensure_part(d, (size_t)P.ns * ni * kResStride);
-    if (rc) return rc;
-    A.out = d->part_d;
-  } else {
-    A.out = res_dev;
-  }
+  A.out = P.ns > 1 ? d->part_d : res_dev;
   CK(d, launch_force(d->order, d->prec, A, P.tpi, P.ip, d->stream));
   const ReduceArgs R{A.out, P.ns, ni, out, A.pred, nj, P.tpi, i_dev, A.iperm, d->status_d,
                      direct ? d->status_h : nullptr};

@@ -7,9 +7,9 @@
 //   force_kernel     i-tile x j-slice Hermite 4th/6th force, nearest
 //                    neighbour and neighbour list
 //                    (role of dev_evaluate_gravity_*, kernels.cu:552-1041)
-//   reduce_kernel    deterministic FP64 sum of the per-slice partials and
-//                    nearest-neighbour min (replaces the FP64 atomics of
-//                    kernels.cu:970-1003)
+//   reduce_kernel    deterministic FP64 sum of the per-slice partials, the
+//                    nearest-neighbour min and its id, looked up once per i
+//                    (replaces the FP64 atomics of kernels.cu:970-1003)
 #pragma once
 #include "sapb_internal.cuh"
 
@@ -60,9 +60,6 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;
