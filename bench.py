@@ -213,12 +213,12 @@ def device_arm(cfg, precision: int, steps: int, warmup: int, torch, flush, lists
     far_tiles, warp_tiles = s.spatial_stats(reset=True)
     s.close()
     spatial = precision == sp.DOUBLESINGLE and warp_tiles > 0
-    # own kernels in the timed steps: predictor, force (+ slice reduction);
+    # own kernels in the timed steps: predictor, force, slice reduction;
     # in spatial mode the j gather, i keys and bounds every step, plus frame
     # init, frame and j keys on the steps that re-sort j (the first call and
     # every 17th after it: the library reuses an order 16 times); the radix
     # sorts are CUB's kernels, not counted
-    per = 2 + (1 if ns > 1 else 0) + (3 if spatial else 0)
+    per = 3 + (3 if spatial else 0)
     timed = range(warmup, warmup + steps)
     launches = per * steps + (3 * sum(1 for c in timed if c % 17 == 0) if spatial else 0)
     return {"pred_ms": pred_ms, "force_ms": force_ms, "comb_ms": comb_ms, "res": out,
