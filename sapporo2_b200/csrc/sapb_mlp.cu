@@ -612,12 +612,21 @@ int sapb_mlp_destroy(sapb_mlp *m) {
   return SAPB_OK;
 }
 
+// Parameters and moments travel on the handle's stream, where the kernels that
+// use them run: the stream is non-blocking, so nothing orders it after a copy or
+// a memset on the default stream (a pageable copy this small returns before it
+// has landed, a memset at once).
 int sapb_mlp_set_params(sapb_mlp *m, const float *params) {
   if (!m || !params) return sapb_fail(m ? m->d : nullptr, SAPB_EINVAL, "bad arguments");
   MK(m, cudaSetDevice(m->d->device));
-  MK(m, cudaMemcpy(m->P, params, sizeof(float) * kNP, cudaMemcpyHostToDevice));
-  MK(m, cudaMemset(m->M, 0, sizeof(float) * kNP));
-  MK(m, cudaMemset(m->V, 0, sizeof(float) * kNP));
+  cudaStream_t st = m->d->stream;
+  MK(m, cudaMemcpyAsync(m->P, params, sizeof(float) * kNP, cudaMemcpyHostToDevice, st));
+  MK(m, cudaMemsetAsync(m->M, 0, sizeof(float) * kNP, st));
+  MK(m, cudaMemsetAsync(m->V, 0, sizeof(float) * kNP, st));
+  // a pageable source has been staged by now, a pinned one may still be read
+  cudaPointerAttributes at{};
+  MK(m, cudaPointerGetAttributes(&at, params));
+  if (at.type != cudaMemoryTypeUnregistered) MK(m, cudaStreamSynchronize(st));
   m->steps = 0;
   return SAPB_OK;
 }
@@ -625,7 +634,9 @@ int sapb_mlp_set_params(sapb_mlp *m, const float *params) {
 int sapb_mlp_get_params(sapb_mlp *m, float *params) {
   if (!m || !params) return sapb_fail(m ? m->d : nullptr, SAPB_EINVAL, "bad arguments");
   MK(m, cudaSetDevice(m->d->device));
-  MK(m, cudaMemcpy(params, m->P, sizeof(float) * kNP, cudaMemcpyDeviceToHost));
+  cudaStream_t st = m->d->stream;
+  MK(m, cudaMemcpyAsync(params, m->P, sizeof(float) * kNP, cudaMemcpyDeviceToHost, st));
+  MK(m, cudaStreamSynchronize(st));
   return SAPB_OK;
 }
 
