@@ -606,6 +606,12 @@ int sapb_push_j(sapb_dev *d, int n) {
   if (!d || n < 0 || n > d->stage_cap) return fail(d, SAPB_EINVAL, "push of %d records", n);
   if (n == 0) return SAPB_OK;
   CK(d, cudaSetDevice(d->device));
+  // A captured push would read the staging at each replay, after the host has
+  // written other records there: refused, before anything is queued.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CK(d, cudaStreamIsCapturing(d->stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+    return fail(d, SAPB_ECUDA, "push of %d records on a stream that is being captured", n);
   // grow the j store to cover the highest staged address
   int maxaddr = -1;
   const int ss = stage_stride(d->order);
