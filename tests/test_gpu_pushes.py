@@ -1,4 +1,6 @@
-"""GPU: a j push is refused on a stream that is being captured."""
+"""GPU: small j pushes, which the scatter kernel reads from one pinned buffer:
+that buffer is not rewritten while a push before it is still queued, and a push
+is refused on a stream that is being captured."""
 import ctypes as C
 
 import numpy as np
@@ -25,6 +27,40 @@ def _positions(s, n):
     out = np.zeros((n, 24))
     assert s.lib.sapb_read_j(s.dev, 0, n, 0.0, 0, out) == 0
     return out[:, 0:3]
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513])
+def test_pushes_behind_a_long_call(gpu, n):
+    """Pushes queued behind a force call of some milliseconds, the staging
+    overwritten after each: none of them has run when the next one comes."""
+    import torch
+    nj, ni = 65536, 65536
+    rng = np.random.default_rng(n)
+    with sp.Sapporo(order=sp.FOURTH, precision=sp.DOUBLE) as s:
+        z = np.zeros((nj, 3))
+        x = rng.normal(size=(nj, 3))
+        s.set_j_particles(np.arange(nj), np.arange(nj), np.zeros(nj), np.ones(nj), x, z, z, z)
+        s.force_prediction(nj)
+        rec = sp.pack_i_records(sp.FOURTH, x[:ni], z[:ni], np.zeros(ni), np.arange(ni), None)
+        stream = torch.cuda.Stream()
+        s.set_stream(stream.cuda_stream)
+        i = torch.from_numpy(rec).cuda()
+        res = torch.zeros(ni, sp.RES_STRIDE, dtype=torch.float64, device="cuda")
+        want = x[:8 * n].copy()
+        torch.cuda.synchronize()
+        assert s.lib.sapb_force_device(s.dev, nj, ni, i.data_ptr(), 1e-6, 0, res.data_ptr(),
+                                       None, None) == 0
+        before = torch.cuda.Event()
+        before.record(stream)
+        for k in range(6):
+            addr = rng.permutation(8 * n)[:n]
+            want[addr] = rng.normal(size=(n, 3))
+            if k == 0 and n <= 512:
+                assert not before.query()
+            assert s.lib.sapb_push_j(s.dev, _stage(s, addr, want[addr])) == 0
+        _stage(s, np.arange(n), np.full((n, 3), np.nan))  # not pushed
+        assert np.array_equal(_positions(s, 8 * n), want)
+        s.set_stream(0)
 
 
 @pytest.mark.parametrize("n", [1, 512, 513])
