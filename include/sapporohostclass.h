@@ -108,6 +108,7 @@ class sapporo {
            int precision = DOUBLESINGLE);
   int close();
   int get_n_pipes();
+  int j_memory() const { return nj_max; }  // addresses below it are accepted as they are
   int set_time(double ti);
   int set_no_time();
 

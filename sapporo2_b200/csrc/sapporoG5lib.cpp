@@ -69,20 +69,19 @@ void g5_set_eps2_to_all(double eps2) { eps_to_use = eps2; }
 void g5_set_eps_to_all(double eps) { eps_to_use = eps * eps; }
 
 void g5_set_xmj(int addr, int nj, double xj[][3], double jmass[]) {
-  // one bulk upload; arrays indexed by address (:111-115), ids = addresses
-  if (nj <= 0) return;
-  if (addr >= 0) {
-    std::vector<int> at((size_t)nj);
-    for (int i = 0; i < nj; i++) at[i] = addr + i;
-    if (grav5.set_j_particles(nj, at.data(), at.data(), nullptr, jmass + addr, xj[addr], nullptr,
-                              nullptr, nullptr, nullptr, nullptr, nullptr) == 0)
-      return;
-  }
-  // refused as a whole (an address beyond the j memory): one by one, as far as
-  // they go
+  // Arrays indexed by address, ids = addresses (:111-115).  Addresses outside the
+  // j memory go one by one, each growing it once or being refused; from the
+  // first one inside, all are accepted and go in one bulk upload.
   double z[3] = {0, 0, 0};
-  for (int i = addr; i < addr + nj; i++)
+  int i = addr;
+  const int end = addr + nj;
+  for (; i < end && (i < 0 || i >= grav5.j_memory()); i++)
     grav5.set_j_particle(i, i, 0.0, 0.0, jmass[i], z, z, z, z, xj[i], z, z, 0.0);
+  if (i >= end) return;
+  std::vector<int> at((size_t)(end - i));
+  for (int k = i; k < end; k++) at[k - i] = k;
+  grav5.set_j_particles(end - i, at.data(), at.data(), nullptr, jmass + i, xj[i], nullptr, nullptr,
+                        nullptr, nullptr, nullptr, nullptr);
 }
 
 void g5_set_jp(int addr, int nj, double jmass[], double xj[][3]) {
