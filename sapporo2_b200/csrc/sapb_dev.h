@@ -60,6 +60,7 @@ struct sapb_dev {
   int i_cap = 0;
   double *res_h = nullptr, *res_d = nullptr;
   int *ngb_count_d = nullptr, *ngb_list_d = nullptr;
+  double *part0_d = nullptr;  // scratch from sapb_open; part_d: grown on demand
   double *part_d = nullptr;
   size_t part_cap = 0;  // doubles
   int *status_d = nullptr, *status_h = nullptr;
