@@ -161,13 +161,19 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // there (reduce_one).  Rescans recompute ds2 bit-identically (same rounded
 // operations).
 // ========================================================================
-// Unroll depth of the packed j loop (B200, 6th order, N = 2^20: 1 -> 501,
-// 2 -> 526, 4 -> 530 G interactions/s).
-#ifndef SAPB_JUNROLL
-#define SAPB_JUNROLL 4
-#endif
-#define SAPB_STR(x) #x
-#define SAPB_UNROLL(n) _Pragma(SAPB_STR(unroll n))
+// Records unrolled in the packed j loop (two i per register pair).  What bounds
+// that loop is the FMA pipe, kept fed by four warps per scheduler at 128
+// registers, so it depends on how the loads and the dependent steps of
+// neighbouring records are interleaved.  6th order: four (N = 2^20: 1 -> 501,
+// 2 -> 526, 4 -> 530 G interactions/s; eight lose up to 2.7 % with four i per
+// thread).  4th order and GRAPE-5, whose body is half as long: full tiles take a
+// loop of constant length, 16 records deep with two i per thread and 8 with four
+// (16 there: up to 28 % slower).  4th order, 60000 x 60000 in address order,
+// from four records at a variable length: (8,2) 4.64 -> 4.46 ms, (4,2) 4.40 ->
+// 4.28, (2,2) 4.24 -> 4.19, (1,2) 4.29 -> 4.24, (2,4) 4.28 -> 4.16, (1,4) 4.20 ->
+// 4.11; 65536 i on 131072 j, spatial mode: 1-2 % with two i per thread.
+template <int ORDER, int IP>
+constexpr int kJUnroll = ORDER >= SIXTH ? 4 : (IP == 4 ? 8 : 16);
 
 template <int ORDER, int PREC, int TPI, int IP>
 __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
@@ -381,28 +387,37 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           far = __all_sync(0xffffffffu, ok);
           nfar += far ? 1 : 0;
         }
+        // this row's records of the tile
+        auto each_record = [&](auto pair) {
+          if (ORDER < SIXTH && cnt == kTJ) {
+            constexpr int JU = kJUnroll<ORDER, IP>;
+#pragma unroll JU
+            for (int k = 0; k < kTJ; k += TPI) pair(k + ty);
+          } else {
+#pragma unroll 4
+            for (int k = ty; k < cnt; k += TPI) pair(k);
+          }
+        };
         // The far loop is written out twice, for calls with and without
         // lists, although both copies are the same: with one shared copy the
         // kernel measured 1.5 % slower on B200, with lists and without (same
         // box, alternating runs).
         if (far && A.do_list) {
-          SAPB_UNROLL(SAPB_JUNROLL)
-          for (int k = ty; k < cnt; k += TPI) {
+          each_record([&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r2 = rec[k * C::RS + 2];
             const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
 #pragma unroll
             for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
-          }
+          });
         } else if (far) {
-          SAPB_UNROLL(SAPB_JUNROLL)
-          for (int k = ty; k < cnt; k += TPI) {
+          each_record([&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r2 = rec[k * C::RS + 2];
             const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
 #pragma unroll
             for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
-          }
+          });
         } else if (ORDER != GRAPE5 && A.list_bits) {
           // 32 records of a row at a time: the list hits are one bit per record
           // (all rows of the warp take every turn, some with no record left)
@@ -412,7 +427,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
             uint2 hit[NPAIR];
 #pragma unroll
             for (int q = 0; q < NPAIR; q++) hit[q] = make_uint2(0u, 0u);
-            SAPB_UNROLL(SAPB_JUNROLL)
+#pragma unroll (ORDER >= SIXTH ? 4 : 8)
             for (int k = k0; k < k1; k += TPI) {
               const float4 r0 = rec[k * C::RS + 0];
               const float4 r1 = rec[k * C::RS + 1];
@@ -433,8 +448,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           }
         } else {
           uint2 none;
-          SAPB_UNROLL(SAPB_JUNROLL)
-          for (int k = ty; k < cnt; k += TPI) {
+          each_record([&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r1 = rec[k * C::RS + 1];
             const float4 r2 = rec[k * C::RS + 2];
@@ -442,7 +456,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
 #pragma unroll
             for (int q = 0; q < NPAIR; q++)
               pair_mix2<ORDER>(I2[q], r0, r1, r2, r3, eps2v, Q[q], tm[q], none, int2{});
-          }
+          });
         }
 #pragma unroll
         for (int q = 0; q < NPAIR; q++) {
