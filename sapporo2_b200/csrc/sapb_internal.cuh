@@ -68,6 +68,7 @@ struct ForceArgs {
   int nslices;        // S: j slices across blocks (slice s: tiles s, s+S, ...)
   int i_tiles;        // number of i tiles
   double *out;        // one 12-double record per (slice, i), see ReduceArgs
+  int finish;         // one slice: `out` holds the results, ids looked up, no reduction
   int do_list;        // build neighbour lists
   int list_bits;      // ... from one bit per record (mixed precision, address order)
   int *ngb_count;     // [ni] (zeroed before launch)

@@ -618,8 +618,18 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
     o[0] = D[p].ax; o[1] = D[p].ay; o[2] = D[p].az; o[3] = D[p].pot;
     o[4] = D[p].jx; o[5] = D[p].jy; o[6] = D[p].jz;
     o[7] = D[p].sx; o[8] = D[p].sy; o[9] = D[p].sz;
-    o[10] = __longlong_as_double((long long)key[p]);
-    o[11] = __longlong_as_double((long long)where[p]);
+    if (A.finish) {
+      if (where[p] != kNnDone) {
+        const unsigned t = (unsigned)(where[p] >> 32);
+        key[p] = nn_scan<ORDER, PREC>(tile_rec(t), tile_cnt(t), (unsigned)where[p], TPI, 0, 1,
+                                      A.irec + (size_t)oi[p] * istr);
+      }
+      o[10] = (double)__uint_as_float((unsigned)(key[p] >> 32));
+      o[11] = (double)(int)(unsigned)key[p];
+    } else {
+      o[10] = __longlong_as_double((long long)key[p]);
+      o[11] = __longlong_as_double((long long)where[p]);
+    }
   }
 }
 
