@@ -272,6 +272,7 @@ constexpr int kSpatialMinJ = 65536;
 struct Shape {
   int tpi, ip;
 };
+constexpr int kMaxSlices = 65535;  // slices are blockIdx.y
 
 // Mixed precision.  The fewer threads per i, the longer the FP32 sums before
 // they are folded to FP64 (256 / TPI records): the acceleration's relative
@@ -368,7 +369,8 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, bool direct = false) {
   const double sm_rate = d->prec == DOUBLE ? (d->order >= SIXTH ? 1.7e9 : 2.4e9)
                                            : (d->order >= SIXTH ? 3.6e9 : 5.6e9);
   // one tile or more per slice; partial records up to 256 MB
-  const int max_ns = (int)std::max(1.0, std::min<double>(ntiles, 268435456.0 / (96.0 * ni)));
+  const int max_ns = (int)std::max(
+      1.0, std::min<double>(std::min(ntiles, kMaxSlices), 268435456.0 / (96.0 * ni)));
   Plan best{1, 2, 1, 1, ntiles};
   double best_t = 1e300;
   const SliceCost cost = d->prec == DOUBLE ? kCostFp64
@@ -398,8 +400,10 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, bool direct = false) {
     }
   };
   if (d->nslices) {
-    const int st = (ntiles + std::min(d->nslices, ntiles) - 1) / std::min(d->nslices, ntiles);
-    consider((ntiles + st - 1) / st);  // every slice non-empty
+    // as the caller asks, in slices of four tiles or more, none empty
+    const int ns = std::min(std::min(d->nslices, std::max(1, ntiles / 4)), kMaxSlices);
+    const int st = (ntiles + ns - 1) / ns;
+    consider((ntiles + st - 1) / st);
   } else {
     // the fewest slices for each length of the longest one
     for (int ns = 1; ns <= max_ns;) {
