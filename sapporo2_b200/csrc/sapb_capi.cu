@@ -292,7 +292,7 @@ constexpr int kMaxSlices = 65535;  // slices are blockIdx.y
 static Shape shape_mixed(const sapb_dev *d, int ni, int nj) {
   static const Shape shapes[] = {{1, 4}, {2, 4}, {1, 2}, {2, 2}, {4, 2}, {8, 2}, {16, 1}, {32, 1}};
   // throughput of a full GPU: 537.8, 534.6, 521.8, 516.1, 510.4 and 491.2 G
-  // interactions/s at N = 2^20, 6th order; the last two are estimates
+  // interactions/s at N = 2^20, 6th order; the last two are estimates for few i
   static const double eff[] = {1.0, 0.994, 0.970, 0.960, 0.949, 0.913, 0.85, 0.85};
   const bool spatial = use_spatial(d, ni, nj);
   // spatial mode asked for at any size: few i take the shapes of address order
@@ -313,7 +313,12 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj) {
   for (int q = first; q <= last; q++) {
     const int ti = force_tile_i(shapes[q].tpi, shapes[q].ip);
     const int i_tiles = std::max(1, (ni + ti - 1) / ti);
-    const int bps = blocks_per_sm(d->order, d->prec, shapes[q].tpi, shapes[q].ip);
+    // the one-i shapes run four blocks on an SM at 6th order, but each does less
+    // than a quarter of one's work (65536 j, 1000 i: (16,1) 178 us, (32,1) 225):
+    // counted as the three they would be with a third stage of tiles
+    const int bps = shapes[q].ip == 1 && d->order >= SIXTH
+                        ? 3
+                        : blocks_per_sm(d->order, d->prec, shapes[q].tpi, shapes[q].ip);
     const long slots = (long)d->num_sms * bps;
     const double tile_time = 128.0 * ti * bps / (eff[q] * sm_rate);
     auto consider = [&](int ns) {
