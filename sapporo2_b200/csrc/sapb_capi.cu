@@ -225,6 +225,9 @@ static int ensure_part(sapb_dev *d, size_t doubles, double **room) {
 struct Plan {
   int tpi, ip, ns, i_tiles, slice_tiles;
 };
+// Where a call's results go: the caller's device buffer; or, for host calls,
+// device memory and a copy, or pinned memory straight from the reduction.
+enum class Call { device, copied, pinned };
 
 // resident blocks per SM of a force-kernel shape (occupancy API)
 static int blocks_per_sm(int order, int prec, int tpi, int ip) {
@@ -280,16 +283,15 @@ constexpr int kMaxSlices = 65535;  // slices are blockIdx.y
 // (16,1), 3.1e-8 with (8,2), 3.2e-8 with (4,2), 3.6e-8 with (2,4) or (2,2) and
 // 5.1e-8 with (1,4).  Time steps of tight binaries follow that rounding, so a
 // shape gives way to a faster one only where that has as many threads per i.
-// (Families with fewer, (8,1) for (32,1) below 1024 i, (4,2) for (8,2) below
-// 8192, (1,4) or (2,4) for all calls in spatial mode, were 1-30 % faster, with
-// errors up to 1.9 times as large.)
+// (Families with fewer below 1024 and 8192 i, (8,1) for (32,1), (4,2) for (8,2),
+// were 1-30 % faster, with errors up to 1.9 times as large.)
 //
 // Free choice among all shapes, or below 2^32 pairs and 2^19 j in address order
 // among those of the call's size (two i per thread with about 65536 / ni
 // threads per i from 1024 i on: 16384 x 16384, 4th order, 0.45 ms against
 // 0.66 for the free choice; 8 or more threads per i below), by the time of whole
 // waves of blocks of four tiles or more, a tile more for a block's start.
-static Shape shape_mixed(const sapb_dev *d, int ni, int nj) {
+static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
   static const Shape shapes[] = {{1, 4}, {2, 4}, {1, 2}, {2, 2}, {4, 2}, {8, 2}, {16, 1}, {32, 1}};
   // throughput of a full GPU: 537.8, 534.6, 521.8, 516.1, 510.4 and 491.2 G
   // interactions/s at N = 2^20, 6th order; the last two are estimates for few i
@@ -343,16 +345,19 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj) {
       if (ns >= 1) consider((int)ns);
     }
   }
-  // Spatial mode: at least four threads per i below 60000 i.  What matters there
-  // is that a block step's calls round alike: the sums of one tile, all in one
-  // direction, err differently with each shape, and the corrector's third
-  // differences amplify the change.  200 block steps of 262144 bodies with tight
-  // binaries, five seeds, t reached in 1e-3: so 3.13, 3.45, 3.85, 0.09 and 0.02;
-  // by the times above alone 3.13, 0.02, 3.57, 0.09 and 0.02; (2,4) throughout
-  // 0.24, 3.27, 3.57, 0.21 and 0.02.  (4,2) is 0-3 % slower there than the
-  // fastest shape.  With (2,4) for (1,4) above, the fourth seed reaches 3.66, but
-  // 500009 x 500009 at 6th order takes 413.6 ms instead of 399.6.
-  if (ordered && ni < 60000 && best.tpi < 4) return {4, 2};
+  // Host calls in spatial mode, below 2^19 j and 60000 i: at least four threads
+  // per i.  Block steps of one system mix calls of all widths, and where shapes
+  // change between them the sums of a tile err differently from step to step,
+  // which the corrector's third differences amplify: 200 block steps of 262144
+  // bodies with tight binaries, eight seeds, reach t > 3e-3 in five with (4,2)
+  // and in three with the fastest shapes (in FP64 in both of those tried).  It
+  // costs 1-2 % at 12983 i on 131072 j and 5-7 % of the force time at 32768 i on
+  // 262144 j, less with the host's share of such a call.  From 2^19 j on, where
+  // the force is all of a call's time, the fastest shape wins (16384 i on 2^20 j,
+  // 6th order: (4,2) 29.6 ms, (1,4) 28.0), as it does for callers with their own
+  // device buffers, who can set a shape.
+  if (call != Call::device && ordered && nj < (1 << 19) && ni < 60000 && best.tpi < 4)
+    return {4, 2};
   return best;
 }
 
@@ -365,8 +370,7 @@ static Shape shape_fp64(int ni, int nj) {
   return ni >= 16384 && nj >= 65536 ? Shape{8, 2} : Shape{8, 1};
 }
 
-// `direct`: results to pinned memory, always through the reduction.
-static Plan make_plan(const sapb_dev *d, int ni, int nj, bool direct = false) {
+static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call) {
   const int tj = force_tile_j();
   const int ntiles = std::max(1, (nj + tj - 1) / tj);
   // pairs per SM and second of a full GPU (B200, order of magnitude): only
@@ -381,7 +385,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, bool direct = false) {
   const SliceCost cost = d->prec == DOUBLE ? kCostFp64
                          : use_spatial(d, ni, nj) ? kCostSpatial : kCostAddress;
   const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
-                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj);
+                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj, call);
   const int tpi = sh.tpi, ip = sh.ip;
   const int ti = force_tile_i(tpi, ip);
   const int i_tiles = (ni + ti - 1) / ti;
@@ -398,7 +402,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, bool direct = false) {
     const double used = std::min<double>(bps, ceil(B / sms)) / bps;
     double t = tiles * sqrt(used) * tile_time;
     if (ns > 1)
-      t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12) + (direct ? 0.0 : kReduceS);
+      t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12) + (call == Call::pinned ? 0.0 : kReduceS);
     if (t < best_t * (best_t < 1e299 ? cost.more : 1.0)) {
       best_t = t;
       best = Plan{tpi, ip, ns, i_tiles, st};
@@ -716,12 +720,13 @@ static float near_r2(const sapb_dev *d, double eps2) {
 // warp's neighbours into a few tiles (8192 i on 131072 j 2.21 against 2.15).
 constexpr int kListBitsMaxJ = 65536;
 
-// `out`: where the results go, res_dev or pinned host memory (`direct`: and the
-// error word to status_h; the list counts are clear already).
+// `out`: where the results go, res_dev or (Call::pinned) pinned host memory, and
+// then the error word to status_h; the list counts are clear already there.
 static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double eps2, int flags,
-                     double *res_dev, int *cnt_dev, int *list_dev, double *out, bool direct) {
+                     double *res_dev, int *cnt_dev, int *list_dev, double *out, Call call) {
   if (nj <= 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
-  Plan P = make_plan(d, ni, nj, direct);
+  const bool direct = call == Call::pinned;
+  Plan P = make_plan(d, ni, nj, call);
   double *part = nullptr;
   if (P.ns > 1) {
     const int rc = ensure_part(d, (size_t)P.ns * ni * kResStride, &part);
@@ -790,7 +795,7 @@ int sapb_force(sapb_dev *d, int nj, int ni, double eps2, double ti, int flags) {
     CK(d, cudaMemcpyAsync(d->irec_d, d->irec_h, sizeof(double) * (size_t)words,
                           cudaMemcpyHostToDevice, d->stream));
     int rc = run_force(d, nj, ni, d->irec_d, eps2, flags, d->res_d, d->ngb_count_d, d->ngb_list_d,
-                       d->res_d, false);
+                       d->res_d, Call::copied);
     if (rc) return rc;
     CK(d, cudaMemcpyAsync(d->res_h, d->res_d, sizeof(double) * kResStride * (size_t)ni,
                           cudaMemcpyDeviceToHost, d->stream));
@@ -807,7 +812,7 @@ int sapb_force(sapb_dev *d, int nj, int ni, double eps2, double ti, int flags) {
     CK(d, launch_predict(d->order, d->prec, predict ? nj : 0, ti, d->js, d->pred, prep, d->stream));
     if (predict) d->pred_gen++;
     int rc = run_force(d, nj, ni, d->irec_d, eps2, flags, d->res_d, d->ngb_count_d, d->ngb_list_d,
-                       d->res_h, true);
+                       d->res_h, Call::pinned);
     if (rc) return rc;
   }
   CK(d, cudaEventRecord(d->done, d->stream));
@@ -856,7 +861,7 @@ int sapb_force_device(sapb_dev *d, int nj, int ni, const double *i_dev, double e
   CK(d, cudaSetDevice(d->device));
   if (ni == 0) return SAPB_OK;
   return run_force(d, nj, ni, i_dev, eps2, flags, res_dev, ngb_count_dev, ngb_list_dev, res_dev,
-                   false);
+                   Call::device);
 }
 
 int sapb_wait_selftest(sapb_dev *d, int limit_ms) {
@@ -894,7 +899,7 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
   double *scratch = g_noalloc_ptr[d->device];
   // Same plan as sapb_force_device, with the j-split capped so that the
   // per-slice partial records fit the fixed scratch.
-  Plan P = make_plan(d, ni, nj);
+  Plan P = make_plan(d, ni, nj, Call::device);
   const int tj = force_tile_j();
   const int ntiles = (nj + tj - 1) / tj;
   const int max_ns = (int)std::max<size_t>(1, cap_records / (size_t)ni);
@@ -973,7 +978,7 @@ int sapb_set_launch(sapb_dev *d, int tpi, int ip, int nslices) {
 
 int sapb_get_plan(sapb_dev *d, int ni, int nj, int *tpi, int *ip, int *nslices) {
   if (!d || ni <= 0 || nj <= 0) return fail(d, SAPB_EINVAL, "bad sizes");
-  const Plan P = make_plan(d, ni, nj);
+  const Plan P = make_plan(d, ni, nj, Call::device);
   if (tpi) *tpi = P.tpi;
   if (ip) *ip = P.ip;
   if (nslices) *nslices = P.ns;
