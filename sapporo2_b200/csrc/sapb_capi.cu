@@ -298,7 +298,8 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
   static const double eff[] = {1.0, 0.994, 0.970, 0.960, 0.949, 0.913, 0.85, 0.85};
   const bool spatial = use_spatial(d, ni, nj);
   // spatial mode asked for at any size: few i take the shapes of address order
-  // (6th order, 1 i on 131072 j, host call: 77 us against 156 with (1,4))
+  // (6th order, 1 i on 131072 j, host call: 77 us against 156 with (1,4)), but
+  // not the one-i ones, whose kernels know no far tiles
   const bool ordered = spatial && ni >= kSpatialMinI && nj >= kSpatialMinJ;
   int first = 0, last = 7;
   if ((double)ni * nj < 4294967296.0 && nj < (1 << 19) && !ordered) {
@@ -307,6 +308,7 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
     first = ni < 1024 ? 5 : (t == 2 ? 3 : (t == 4 ? 4 : 5));
     if (ni >= 1024) last = first;
   }
+  if (spatial) last = std::min(last, 5);
   const int tj = force_tile_j(), ntiles = std::max(1, (nj + tj - 1) / tj);
   const int max_ns = std::max(1, ntiles / 4);
   const double sm_rate = d->order >= SIXTH ? 3.6e9 : 5.6e9;
@@ -739,7 +741,8 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
   if (list && !direct) CK(d, cudaMemsetAsync(cnt_dev, 0, sizeof(int) * (size_t)ni, d->stream));
   ForceArgs A{};
   A.pred = d->pred;
-  bool spatial = use_spatial(d, ni, nj);
+  // (one-i shapes set by the caller ignore the boxes: nothing to prepare)
+  bool spatial = use_spatial(d, ni, nj) && P.ip % 2 == 0;
   if (spatial) {
     const int rc = spatial_prepare(d, nj, ni, i_dev);
     if (rc == SAPB_ENOMEM) spatial = false;  // no room for its buffers: address order
