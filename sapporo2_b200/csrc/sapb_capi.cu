@@ -247,11 +247,20 @@ static int blocks_per_sm(int order, int prec, int tpi, int ip) {
 // its records to the reduction, and kSliceS to that kernel's chain of loads.
 // More slices are taken only where they cost less than `more` of fewer: other
 // calls on the GPU pay for every block's start.
+//
+// The constants are a compromise between a call alone and calls of three
+// streams back to back, over 44 calls from 1024 x 1024 to 16384 i on 2^20 j with
+// 1 to 64 slices each: back to back within 1 % of the best number on average
+// (2.7 % at most), alone within 2.2 %.  Smaller ones favour the call alone and
+// take up to four times the slices: with block 0.3 and tail 0.6, 5000 i on
+// 65536 j at 4th order ran in 22 slices, 398 us back to back and 522 alone,
+// against 378 and 551 in 7; 8192 x 8192 at 6th order in 5, 148 and 200 against
+// 142 and 213 in 3.
 struct SliceCost {
   double block, tail, more;
 };
-constexpr SliceCost kCostAddress{0.3, 0.6, 0.96};
-constexpr SliceCost kCostSpatial{0.3, 0.6, 1.0 - 1e-9};
+constexpr SliceCost kCostAddress{1.0, 0.45, 0.97};
+constexpr SliceCost kCostSpatial{1.0, 1.0, 1.0 - 1e-9};  // near tiles run longer: whole waves
 constexpr SliceCost kCostFp64{0.3, 0.6, 0.99};
 constexpr double kSliceS = 5e-8;
 // A call with one slice on the device's own buffers launches no reduction
