@@ -169,9 +169,12 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // thread).  4th order and GRAPE-5, whose body is half as long: full tiles take a
 // loop of constant length, 16 records deep with two i per thread and 8 with four
 // (16 there: up to 28 % slower).  4th order, 60000 x 60000 in address order,
-// from four records at a variable length: (8,2) 4.64 -> 4.46 ms, (4,2) 4.40 ->
+// from four records at a variable length: (8,2) 4.64 -> 4.48 ms, (4,2) 4.40 ->
 // 4.28, (2,2) 4.24 -> 4.19, (1,2) 4.29 -> 4.24, (2,4) 4.28 -> 4.16, (1,4) 4.20 ->
-// 4.11; 65536 i on 131072 j, spatial mode: 1-2 % with two i per thread.
+// 4.11; GRAPE-5, 65536 i on 131072 j, spatial, 0-4 %.  Not at 4th order in
+// spatial mode: a warp there goes back and forth between far tiles, near tiles
+// and list scans, and with the long loops that is too much code to stay near
+// (8192 i on 131072 j with lists, (2,4) 1.36 -> 1.46 ms).
 template <int ORDER, int IP>
 constexpr int kJUnroll = ORDER >= SIXTH ? 4 : (IP == 4 ? 8 : 16);
 
@@ -387,9 +390,9 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           far = __all_sync(0xffffffffu, ok);
           nfar += far ? 1 : 0;
         }
-        // this row's records of the tile
-        auto each_record = [&](auto pair) {
-          if (ORDER < SIXTH && cnt == kTJ) {
+        // this row's records of the tile (`whole`: a full one in the long loop)
+        auto each_record = [&](bool whole, auto pair) {
+          if (ORDER < SIXTH && whole && cnt == kTJ) {
             constexpr int JU = kJUnroll<ORDER, IP>;
 #pragma unroll JU
             for (int k = 0; k < kTJ; k += TPI) pair(k + ty);
@@ -403,7 +406,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
         // kernel measured 1.5 % slower on B200, with lists and without (same
         // box, alternating runs).
         if (far && A.do_list) {
-          each_record([&](int k) {
+          each_record(ORDER == GRAPE5, [&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r2 = rec[k * C::RS + 2];
             const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
             for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
           });
         } else if (far) {
-          each_record([&](int k) {
+          each_record(ORDER == GRAPE5, [&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r2 = rec[k * C::RS + 2];
             const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           }
         } else {
           uint2 none;
-          each_record([&](int k) {
+          each_record(ORDER == GRAPE5 || !spatial, [&](int k) {
             const float4 r0 = rec[k * C::RS + 0];
             const float4 r1 = rec[k * C::RS + 1];
             const float4 r2 = rec[k * C::RS + 2];
