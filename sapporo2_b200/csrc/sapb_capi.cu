@@ -373,11 +373,17 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
 }
 
 // FP64: one i per thread, four blocks per SM (50021 x 50021, 6th order, (8,2)
-// at three blocks 10.00 ms a pass, (8,1) 9.87).  Calls from 16384 i on 65536 j
-// keep (8,2), the family the planner's test fixes there; (8,1) measured 8.67 ms
+// at three blocks 10.00 ms a pass, (8,1) 9.87).  (16,1) below 1000 i, where it
+// is up to 6 % faster in a call alone (999 i on 32768 j, 6th order, 181 us
+// against 192; 136 against 131 beside other calls) and alike on fewer j; below
+// 4096 x 4096, where it needs one slice and no reduction ((16,1) 36 us and 65
+// alone at 2518 x 2518, 4th order, (8,1) 39 and 59, 77 in one slice); and below
+// 2500 i on at most 16384 j, the family that the planner's test fixes at 2048 x
+// 16384 (4th order (16,1) 100 us, 143 alone; (8,1) 92 and 141).  Calls from
+// 16384 i on 65536 j keep (8,2), fixed there as well; (8,1) measured 8.67 ms
 // against 8.93 at 16384 x 131072.
 static Shape shape_fp64(int ni, int nj) {
-  if (ni < 1000 || (ni < 2500 && nj <= 16384)) return {16, 1};
+  if (ni < 1000 || (ni < 2500 && nj <= 16384) || (ni < 4096 && nj < 4096)) return {16, 1};
   return ni >= 16384 && nj >= 65536 ? Shape{8, 2} : Shape{8, 1};
 }
 
@@ -401,7 +407,10 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call) {
   const int ti = force_tile_i(tpi, ip);
   const int i_tiles = (ni + ti - 1) / ti;
   const int bps = blocks_per_sm(d->order, d->prec, tpi, ip);
-  const double tile_time = (double)tj * ti * bps / sm_rate;
+  // a one-i shape of mixed precision has less arithmetic to hide a tile's loads
+  // and folds behind (60000 x 60000: (16,1) 6.4 ms, (32,1) 8.2, (2,2) 4.2)
+  const double slow = d->prec == DOUBLE || ip > 1 ? 1.0 : (tpi < 32 ? 1.45 : 1.85);
+  const double tile_time = slow * (double)tj * ti * bps / sm_rate;
   auto consider = [&](int ns) {
     const int st = (ntiles + ns - 1) / ns;  // tiles of the longest slice
     const double B = (double)i_tiles * ns, sms = d->num_sms, w = B / (sms * bps);
