@@ -248,17 +248,19 @@ static int blocks_per_sm(int order, int prec, int tpi, int ip) {
 // More slices are taken only where they cost less than `more` of fewer: other
 // calls on the GPU pay for every block's start.
 //
-// The constants are a compromise between a call alone and calls of three
-// streams back to back, over 44 calls from 1024 x 1024 to 16384 i on 2^20 j with
-// 1 to 64 slices each: back to back within 1 % of the best number on average
-// (2.7 % at most), alone within 2.2 %.  Smaller ones favour the call alone and
-// take up to four times the slices: with block 0.3 and tail 0.6, 5000 i on
-// 65536 j at 4th order ran in 22 slices, 398 us back to back and 522 alone,
-// against 378 and 551 in 7; 8192 x 8192 at 6th order in 5, 148 and 200 against
-// 142 and 213 in 3.
+// Host calls wait for their results and have the GPU to themselves: kAlone.
+// Device-resident ones may run beside others: for them the constants are a
+// compromise between a call alone and calls of three streams back to back, over
+// 44 calls from 1024 x 1024 to 16384 i on 2^20 j with 1 to 64 slices each: back
+// to back within 1 % of the best number on average (2.7 % at most), alone within
+// 2.2 %.  With kAlone's they took up to four times the slices: 5000 i on 65536 j
+// at 4th order ran in 22, 398 us back to back and 522 alone, against 378 and 551
+// in 7; 8192 x 8192 at 6th order in 5, 148 and 200 against 142 and 213 in 3.
 struct SliceCost {
   double block, tail, more;
 };
+constexpr SliceCost kAloneAddress{0.3, 0.6, 0.96};
+constexpr SliceCost kAloneSpatial{0.3, 0.6, 1.0 - 1e-9};
 constexpr SliceCost kCostAddress{1.0, 0.45, 0.97};
 constexpr SliceCost kCostSpatial{1.0, 1.0, 1.0 - 1e-9};  // near tiles run longer: whole waves
 constexpr SliceCost kCostFp64{0.3, 0.6, 0.99};
@@ -399,8 +401,10 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call) {
       1.0, std::min<double>(std::min(ntiles, kMaxSlices), 268435456.0 / (96.0 * ni)));
   Plan best{1, 2, 1, 1, ntiles};
   double best_t = 1e300;
+  const bool spatial = use_spatial(d, ni, nj), alone = call != Call::device;
   const SliceCost cost = d->prec == DOUBLE ? kCostFp64
-                         : use_spatial(d, ni, nj) ? kCostSpatial : kCostAddress;
+                         : spatial         ? (alone ? kAloneSpatial : kCostSpatial)
+                                           : (alone ? kAloneAddress : kCostAddress);
   const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
                           : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj, call);
   const int tpi = sh.tpi, ip = sh.ip;
