@@ -302,7 +302,7 @@ constexpr int kMaxSlices = 65535;  // slices are blockIdx.y
 // threads per i from 1024 i on: 16384 x 16384, 4th order, 0.45 ms against
 // 0.66 for the free choice; 8 or more threads per i below), by the time of whole
 // waves of blocks of four tiles or more, a tile more for a block's start.
-static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
+static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call, bool lists) {
   static const Shape shapes[] = {{1, 4}, {2, 4}, {1, 2}, {2, 2}, {4, 2}, {8, 2}, {16, 1}, {32, 1}};
   // throughput of a full GPU: 537.8, 534.6, 521.8, 516.1, 510.4 and 491.2 G
   // interactions/s at N = 2^20, 6th order; the last two are estimates for few i
@@ -368,8 +368,12 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call) {
   // 262144 j, less with the host's share of such a call.  From 2^19 j on, where
   // the force is all of a call's time, the fastest shape wins (16384 i on 2^20 j,
   // 6th order: (4,2) 29.6 ms, (1,4) 28.0), as it does for callers with their own
-  // device buffers, who can set a shape.
-  if (call != Call::device && ordered && nj < (1 << 19) && ni < 60000 && best.tpi < 4)
+  // device buffers, who can set a shape; with lists, whose scans weigh on near
+  // tiles, (4,2) is within 1.4 % of it up to 2^31 pairs, and ahead at 8192 i on
+  // 131072 j, 6th order (2.13 ms, (2,4) 2.16), and stays.
+  const bool four = call != Call::device ? nj < (1 << 19)
+                                         : lists && (double)ni * nj < 2147483648.0;
+  if (four && ordered && ni < 60000 && best.tpi < 4)
     return {4, 2};
   return best;
 }
@@ -389,7 +393,7 @@ static Shape shape_fp64(int ni, int nj) {
   return ni >= 16384 && nj >= 65536 ? Shape{8, 2} : Shape{8, 1};
 }
 
-static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call) {
+static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call, bool lists) {
   const int tj = force_tile_j();
   const int ntiles = std::max(1, (nj + tj - 1) / tj);
   // pairs per SM and second of a full GPU (B200, order of magnitude): only
@@ -406,7 +410,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call) {
                          : spatial         ? (alone ? kAloneSpatial : kCostSpatial)
                                            : (alone ? kAloneAddress : kCostAddress);
   const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
-                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj, call);
+                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj, call, lists);
   const int tpi = sh.tpi, ip = sh.ip;
   const int ti = force_tile_i(tpi, ip);
   const int i_tiles = (ni + ti - 1) / ti;
@@ -750,7 +754,8 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
                      double *res_dev, int *cnt_dev, int *list_dev, double *out, Call call) {
   if (nj <= 0 || nj > d->cap) return fail(d, SAPB_EINVAL, "nj = %d (capacity %d)", nj, d->cap);
   const bool direct = call == Call::pinned;
-  Plan P = make_plan(d, ni, nj, call);
+  const bool list = (flags & SAPB_F_NGB_LIST) != 0;
+  Plan P = make_plan(d, ni, nj, call, list);
   double *part = nullptr;
   if (P.ns > 1) {
     const int rc = ensure_part(d, (size_t)P.ns * ni * kResStride, &part);
@@ -759,7 +764,6 @@ static int run_force(sapb_dev *d, int nj, int ni, const double *i_dev, double ep
     if (rc && (rc != SAPB_ENOMEM || d->nslices)) return rc;
     if (rc) P.ns = 1;
   }
-  const bool list = (flags & SAPB_F_NGB_LIST) != 0;
   if (list && !direct) CK(d, cudaMemsetAsync(cnt_dev, 0, sizeof(int) * (size_t)ni, d->stream));
   ForceArgs A{};
   A.pred = d->pred;
@@ -924,7 +928,8 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
   double *scratch = g_noalloc_ptr[d->device];
   // Same plan as sapb_force_device, with the j-split capped so that the
   // per-slice partial records fit the fixed scratch.
-  Plan P = make_plan(d, ni, nj, Call::device);
+  const bool list = (flags & SAPB_F_NGB_LIST) != 0;
+  Plan P = make_plan(d, ni, nj, Call::device, list);
   const int tj = force_tile_j();
   const int ntiles = (nj + tj - 1) / tj;
   const int max_ns = (int)std::max<size_t>(1, cap_records / (size_t)ni);
@@ -932,7 +937,6 @@ int sapb_force_device_noalloc(sapb_dev *d, int nj, int ni, const double *i_dev, 
     P.slice_tiles = (ntiles + max_ns - 1) / max_ns;
     P.ns = (ntiles + P.slice_tiles - 1) / P.slice_tiles;
   }
-  const bool list = (flags & SAPB_F_NGB_LIST) != 0;
   if (list) CK(d, cudaMemsetAsync(ngb_count_dev, 0, sizeof(int) * (size_t)ni, d->stream));
   ForceArgs A{};
   A.pred = d->pred;
@@ -1003,7 +1007,7 @@ int sapb_set_launch(sapb_dev *d, int tpi, int ip, int nslices) {
 
 int sapb_get_plan(sapb_dev *d, int ni, int nj, int *tpi, int *ip, int *nslices) {
   if (!d || ni <= 0 || nj <= 0) return fail(d, SAPB_EINVAL, "bad sizes");
-  const Plan P = make_plan(d, ni, nj, Call::device);
+  const Plan P = make_plan(d, ni, nj, Call::device, false);
   if (tpi) *tpi = P.tpi;
   if (ip) *ip = P.ip;
   if (nslices) *nslices = P.ns;
