@@ -175,8 +175,28 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // spatial mode: a warp there goes back and forth between far tiles, near tiles
 // and list scans, and with the long loops that is too much code to stay near
 // (8192 i on 131072 j with lists, (2,4) 1.36 -> 1.46 ms).
-template <int ORDER, int IP>
-constexpr int kJUnroll = ORDER >= SIXTH ? 4 : (IP == 4 ? 8 : 16);
+// Record k of a tile against a thread's NP pairs of i.
+template <int ORDER, int RS, int NP>
+__device__ __forceinline__ void near_record(const float4 *rec, int k, const IMix2 *I2, float2 eps2,
+                                            AccMix2 *Q, float2 *tm) {
+  const float4 r0 = rec[k * RS + 0];
+  const float4 r1 = rec[k * RS + 1];
+  const float4 r2 = rec[k * RS + 2];
+  const float4 r3 = ORDER >= SIXTH ? rec[k * RS + 3] : r2;
+  uint2 none;
+#pragma unroll
+  for (int q = 0; q < NP; q++)
+    pair_mix2<ORDER>(I2[q], r0, r1, r2, r3, eps2, Q[q], tm[q], none, int2{});
+}
+template <int ORDER, int RS, int NP>
+__device__ __forceinline__ void far_record(const float4 *rec, int k, const IMix2 *I2, float2 eps2,
+                                           AccMix2 *Q) {
+  const float4 r0 = rec[k * RS + 0];
+  const float4 r2 = rec[k * RS + 2];
+  const float4 r3 = ORDER >= SIXTH ? rec[k * RS + 3] : r2;
+#pragma unroll
+  for (int q = 0; q < NP; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2, Q[q]);
+}
 
 template <int ORDER, int PREC, int TPI, int IP>
 __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
@@ -390,11 +410,12 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
           far = __all_sync(0xffffffffu, ok);
           nfar += far ? 1 : 0;
         }
-        // this row's records of the tile (`whole`: a full one in the long loop)
-        auto each_record = [&](bool whole, auto pair) {
-          if (ORDER < SIXTH && whole && cnt == kTJ) {
-            constexpr int JU = kJUnroll<ORDER, IP>;
-#pragma unroll JU
+        // Up to 4th order: this row's records of the tile (`whole`: a full one in
+        // the long loop).  At 6th order the loop is written where it runs: through
+        // here (1,4) lost 0.4 % in spatial mode.
+        [[maybe_unused]] auto each_record = [&](bool whole, auto pair) {
+          if (whole && cnt == kTJ) {
+#pragma unroll (IP == 4 ? 8 : 16)
             for (int k = 0; k < kTJ; k += TPI) pair(k + ty);
           } else {
 #pragma unroll 4
@@ -406,21 +427,25 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
         // kernel measured 1.5 % slower on B200, with lists and without (same
         // box, alternating runs).
         if (far && A.do_list) {
-          each_record(ORDER == GRAPE5, [&](int k) {
-            const float4 r0 = rec[k * C::RS + 0];
-            const float4 r2 = rec[k * C::RS + 2];
-            const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
-#pragma unroll
-            for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
-          });
+          if constexpr (ORDER >= SIXTH) {
+#pragma unroll 4
+            for (int k = ty; k < cnt; k += TPI)
+              far_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q);
+          } else {
+            each_record(ORDER == GRAPE5, [&](int k) {
+              far_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q);
+            });
+          }
         } else if (far) {
-          each_record(ORDER == GRAPE5, [&](int k) {
-            const float4 r0 = rec[k * C::RS + 0];
-            const float4 r2 = rec[k * C::RS + 2];
-            const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
-#pragma unroll
-            for (int q = 0; q < NPAIR; q++) pair_mix2_far<ORDER>(I2[q], r0, r2, r3, eps2v, Q[q]);
-          });
+          if constexpr (ORDER >= SIXTH) {
+#pragma unroll 4
+            for (int k = ty; k < cnt; k += TPI)
+              far_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q);
+          } else {
+            each_record(ORDER == GRAPE5, [&](int k) {
+              far_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q);
+            });
+          }
         } else if (ORDER != GRAPE5 && A.list_bits) {
           // 32 records of a row at a time: the list hits are one bit per record
           // (all rows of the warp take every turn, some with no record left)
@@ -450,16 +475,15 @@ __global__ void __launch_bounds__(kBT, (FCfg<ORDER, PREC, TPI, IP>::MIN_BLOCKS))
             }
           }
         } else {
-          uint2 none;
-          each_record(ORDER == GRAPE5 || !spatial, [&](int k) {
-            const float4 r0 = rec[k * C::RS + 0];
-            const float4 r1 = rec[k * C::RS + 1];
-            const float4 r2 = rec[k * C::RS + 2];
-            const float4 r3 = ORDER >= SIXTH ? rec[k * C::RS + 3] : r2;
-#pragma unroll
-            for (int q = 0; q < NPAIR; q++)
-              pair_mix2<ORDER>(I2[q], r0, r1, r2, r3, eps2v, Q[q], tm[q], none, int2{});
-          });
+          if constexpr (ORDER >= SIXTH) {
+#pragma unroll 4
+            for (int k = ty; k < cnt; k += TPI)
+              near_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q, tm);
+          } else {
+            each_record(ORDER == GRAPE5 || !spatial, [&](int k) {
+              near_record<ORDER, C::RS, NPAIR>(rec, k, I2, eps2v, Q, tm);
+            });
+          }
         }
 #pragma unroll
         for (int q = 0; q < NPAIR; q++) {
