@@ -134,11 +134,12 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // Block = 4 warps, laid out as TPI rows x TIT = 128/TPI columns; each thread
 // owns IP i-particles (columns tx, tx+TIT, ...), so a block covers an i-tile
 // of TI = TIT*IP particles.  blockIdx.y selects j-slice s of S: the tiles
-// s, s+S, s+2S, ... of kTJ = 256 records.  Lane 0 of warp 0 streams them
-// into a 3-stage shared-memory ring with cp.async.bulk (TMA engine): `full`
-// mbarriers signal arrival (complete_tx), and the warp that releases a stage
-// last refills it; there is no block-wide barrier per tile and no warp waits
-// for another one's release, so warps drift up to two tiles apart.
+// s, s+S, s+2S, ... of kTJ = 256 records, streamed into a shared-memory ring of
+// three stages (two where FCfg says why) with cp.async.bulk (TMA engine): thread
+// 0 fills the ring, then the warp that releases a stage last refills it.  `full`
+// mbarriers signal arrival (complete_tx); there is no block-wide barrier per tile
+// and no warp waits for another one's release, so warps drift up to a ring's
+// length apart.
 // Row `ty` consumes records ty, ty+TPI, ... of each tile.
 //
 // Mixed precision (DOUBLESINGLE): dr = (xj_hi - xi_hi) + (xj_lo - xi_lo)
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // more ALU operations per pair keep one bit per record and the warp gathers
 // the set bits after every 32 records.  Nearest neighbour: each thread remembers the tile
 // where its smallest ds2 first appeared, and the reduction looks up the id
-// there (reduce_one).  Rescans recompute ds2 bit-identically (same rounded
+// there (reduce_one), or the i's thread itself in calls that need no reduction
+// (A.finish).  Rescans recompute ds2 bit-identically (same rounded
 // operations).
 // ========================================================================
 // Records unrolled in the packed j loop (two i per register pair).  What bounds
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(256) readj_kernel(int first, int n, double ti,
 // spatial mode: a warp there goes back and forth between far tiles, near tiles
 // and list scans, and with the long loops that is too much code to stay near
 // (8192 i on 131072 j with lists, (2,4) 1.36 -> 1.46 ms).
+
 // Record k of a tile against a thread's NP pairs of i.
 template <int ORDER, int RS, int NP>
 __device__ __forceinline__ void near_record(const float4 *rec, int k, const IMix2 *I2, float2 eps2,

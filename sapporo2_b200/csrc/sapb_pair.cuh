@@ -637,7 +637,7 @@ __device__ __forceinline__ void list_rescan_dp(const IDp &I, bool want, int gi, 
 // ---------------- nearest neighbour ----------------
 // The pair loops keep, per thread and i, only the smallest ds2 and the tile
 // it first appeared in.  Which record that was is looked up once per i, in
-// the reduction over the slices (nn_scan, one warp per i), and not at the end
+// the reduction over the slices (nn_scan, 8 or 32 lanes per i), and not at the end
 // of every slice, where each thread walked its own tile from L2, one record
 // after another (B200, a pass with and without: 192 clusters in a batch
 // 2.45 / 2.72 ms, 12983 i on 131072 j 3.96 / 4.06 ms, 600 i on 30011 j 114 /
