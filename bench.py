@@ -44,8 +44,8 @@ METRIC = "interactions/s at N=2^20 mixed vs plain FP64, 1 GPU, acc err<=1e-6; %F
 # with --spatial 0), and the hash of the kernel sources that capture ran
 # (kernel_source_sha).  When the sources change the figure is stale and the
 # bench reports no traffic until it is captured again.
-FORCE_DRAM = {"source_sha": "94351db47c9b653e",
-              "spatial": 1146223360.0 + 106513408.0, "address": 1011926784.0 + 177736448.0}
+FORCE_DRAM = {"source_sha": "d34af62283c9d458",
+              "spatial": 1150717696.0 + 108259584.0, "address": 989864704.0 + 105665536.0}
 KERNEL_SOURCES = ["sapb_kernels.cu", "sapb_kernels.cuh", "sapb_pair.cuh", "sapb_internal.cuh",
                   "sapb_spatial.cu", "sapb_capi.cu"]
 
@@ -213,12 +213,12 @@ def device_arm(cfg, precision: int, steps: int, warmup: int, torch, flush, lists
     far_tiles, warp_tiles = s.spatial_stats(reset=True)
     s.close()
     spatial = precision == sp.DOUBLESINGLE and warp_tiles > 0
-    # own kernels in the timed steps: predictor, force, slice reduction;
-    # in spatial mode the j gather, i keys and bounds every step, plus frame
-    # init, frame and j keys on the steps that re-sort j (the first call and
-    # every 17th after it: the library reuses an order 16 times); the radix
-    # sorts are CUB's kernels, not counted
-    per = 3 + (3 if spatial else 0)
+    # own kernels in the timed steps: predictor, force, slice reduction (none for
+    # one slice with 8 threads per i or more); in spatial mode the j gather, i
+    # keys and bounds every step, plus frame init, frame and j keys on the steps
+    # that re-sort j (the first call and every 17th after it: the library reuses
+    # an order 16 times); the radix sorts are CUB's kernels, not counted
+    per = (2 if ns == 1 and tpi >= 8 else 3) + (3 if spatial else 0)
     timed = range(warmup, warmup + steps)
     launches = per * steps + (3 * sum(1 for c in timed if c % 17 == 0) if spatial else 0)
     return {"pred_ms": pred_ms, "force_ms": force_ms, "comb_ms": comb_ms, "res": out,

@@ -89,9 +89,8 @@ int sapb_j_stage_stride(const sapb_dev *d);
 /* Copies the first n staged records to the device and scatters them to their
  * addresses.  Up to 512 records the call returns at once and the staging may be
  * written again; more are waited for.  Not on a stream that is being captured.
- * The n records name distinct addresses: of two
- * records for one address either may land.  The sapporo class keeps one
- * record per address, the later values overwriting the earlier, as the
+ * The n records name distinct addresses: of two records for one address either
+ * may land.  The sapporo class keeps one record per address, the later values overwriting the earlier, as the
  * reference's address map does (lib/src/sapporohostclass.cpp:476-494).
  * Replaces send_j_particles_to_device + copyJInDev
  * (lib/src/sapporohostclass.cpp:889-923, 1204-1248). */
@@ -240,7 +239,8 @@ int sapb_mlp_train(sapb_mlp *m, int n, const float *x, const float *t, int epoch
 /* Launch-shape override for the force kernel: threads per i (1,2,4,8,16,32),
  * i per thread (1,2; 4 in mixed precision with 1 or 2 threads per i) and j slices
  * (>= 1; cut to a quarter of the 256-record j tiles).  Zeros restore the built-in
- * planner; sapb_get_plan gives its plan for sapb_force_device without lists.  Replaces the compile-time NTHREADS / NBLOCKS_PER_MULTI tables
+ * planner; sapb_get_plan gives its plan for sapb_force_device without lists.
+ * Replaces the compile-time NTHREADS / NBLOCKS_PER_MULTI tables
  * (lib/include/defines.h:13-122). */
 int sapb_set_launch(sapb_dev *d, int tpi, int ip, int nslices);
 int sapb_get_plan(sapb_dev *d, int ni, int nj, int *tpi, int *ip, int *nslices);
