@@ -90,8 +90,9 @@ int sapb_j_stage_stride(const sapb_dev *d);
  * addresses.  Up to 512 records the call returns at once and the staging may be
  * written again; more are waited for.  Not on a stream that is being captured.
  * The n records name distinct addresses: of two records for one address either
- * may land.  The sapporo class keeps one record per address, the later values overwriting the earlier, as the
- * reference's address map does (lib/src/sapporohostclass.cpp:476-494).
+ * may land.  The sapporo class keeps one record per address, the later values
+ * overwriting the earlier, as the reference's address map does
+ * (lib/src/sapporohostclass.cpp:476-494).
  * Replaces send_j_particles_to_device + copyJInDev
  * (lib/src/sapporohostclass.cpp:889-923, 1204-1248). */
 int sapb_push_j(sapb_dev *d, int n);

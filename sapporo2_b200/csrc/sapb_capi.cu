@@ -387,8 +387,11 @@ static Shape shape_mixed(const sapb_dev *d, int ni, int nj, Call call, bool list
 // 2500 i on at most 16384 j, the family that the planner's test fixes at 2048 x
 // 16384 (4th order (16,1) 100 us, 143 alone; (8,1) 92 and 141).  Calls from
 // 16384 i on 65536 j keep (8,2), fixed there as well; (8,1) measured 8.67 ms
-// against 8.93 at 16384 x 131072.
-static Shape shape_fp64(int ni, int nj) {
+// against 8.93 at 16384 x 131072.  The largest 6th-order calls, 65536 i and 2^32
+// pairs on, take (2,2): 262144 x 262144 265.5 ms, (8,2) 274.0, (8,1) 271.1; at 4th
+// order (8,2) is as fast.
+static Shape shape_fp64(int order, int ni, int nj) {
+  if (order >= SIXTH && ni >= 65536 && (double)ni * nj >= 4294967296.0) return {2, 2};
   if (ni < 1000 || (ni < 2500 && nj <= 16384) || (ni < 4096 && nj < 4096)) return {16, 1};
   return ni >= 16384 && nj >= 65536 ? Shape{8, 2} : Shape{8, 1};
 }
@@ -410,7 +413,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call, bool lists) 
                          : spatial         ? (alone ? kAloneSpatial : kCostSpatial)
                                            : (alone ? kAloneAddress : kCostAddress);
   const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
-                          : d->prec == DOUBLE ? shape_fp64(ni, nj) : shape_mixed(d, ni, nj, call, lists);
+                          : d->prec == DOUBLE ? shape_fp64(d->order, ni, nj) : shape_mixed(d, ni, nj, call, lists);
   const int tpi = sh.tpi, ip = sh.ip;
   const int ti = force_tile_i(tpi, ip);
   const int i_tiles = (ni + ti - 1) / ti;

@@ -1,5 +1,5 @@
-"""GPU: launch shapes that the planner picks for device-resident calls of mixed
-precision, where another family was measured slower."""
+"""GPU: launch shapes that the planner picks for device-resident calls where
+another family was measured slower."""
 import pytest
 
 import sapporo2_b200 as sp
@@ -16,3 +16,9 @@ pytestmark = pytest.mark.gpu
 def test_shapes(gpu, order, ni, nj, shapes):
     with sp.Sapporo(order=order, precision=sp.DOUBLESINGLE) as s:
         assert s.plan(ni, nj)[:2] in shapes
+
+
+@pytest.mark.parametrize("ni,nj", [(65536, 65536), (262144, 262144), (1 << 20, 1 << 20)])
+def test_large_fp64_calls(gpu, ni, nj):
+    with sp.Sapporo(order=sp.SIXTH, precision=sp.DOUBLE) as s:
+        assert s.plan(ni, nj)[:2] == (2, 2)  # (8, 2): 3 % slower at 262144 x 262144
