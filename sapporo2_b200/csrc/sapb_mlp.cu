@@ -620,6 +620,11 @@ int sapb_mlp_set_params(sapb_mlp *m, const float *params) {
   if (!m || !params) return sapb_fail(m ? m->d : nullptr, SAPB_EINVAL, "bad arguments");
   MK(m, cudaSetDevice(m->d->device));
   cudaStream_t st = m->d->stream;
+  // captured, the copy would read `params` at each replay
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  MK(m, cudaStreamIsCapturing(st, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+    return sapb_fail(m->d, SAPB_ECUDA, "network parameters set on a stream that is being captured");
   MK(m, cudaMemcpyAsync(m->P, params, sizeof(float) * kNP, cudaMemcpyHostToDevice, st));
   MK(m, cudaMemsetAsync(m->M, 0, sizeof(float) * kNP, st));
   MK(m, cudaMemsetAsync(m->V, 0, sizeof(float) * kNP, st));

@@ -38,3 +38,26 @@ def test_parameters_do_not_wait_for_the_default_stream(gpu, n):
         assert not busy.query()  # nothing above went through the default stream
         torch.cuda.synchronize()
         net.close()
+
+
+def test_parameters_under_capture_are_refused(gpu):
+    import torch
+
+    import sapporo2_b200 as sp
+    from sapporo2_b200.learned_h2 import H2Net
+    with sp.Sapporo(order=sp.SIXTH) as s:
+        net = H2Net(s, seed=3)
+        p = net.params()
+        stream = torch.cuda.Stream()
+        s.set_stream(stream.cuda_stream)
+        graph = torch.cuda.CUDAGraph()
+        one = torch.zeros(1, device="cuda")
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            one += 1
+            with pytest.raises(sp.SapporoError):
+                net.set_params(p * 2)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(net.params(), p)
+        s.set_stream(0)
+        net.close()
