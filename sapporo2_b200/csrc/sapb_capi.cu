@@ -267,7 +267,10 @@ constexpr SliceCost kCostFp64{0.3, 0.6, 0.99};
 constexpr double kSliceS = 5e-8;
 // A call with one slice on the device's own buffers launches no reduction
 // (run_force): that kernel's launch, its wait for the force kernel and its run.
-constexpr double kReduceS = 1e-5;
+// (Mixed, 6th order, 1024 x 1024: one slice 45 us a pass, 58 alone, four 48 and
+// 58; FP64 keeps the smaller figure, with 12 us 8192 x 8192 at 4th order would go
+// from 8 slices to one, 186 -> 176 us beside other calls but 232 -> 262 alone.)
+constexpr double kReduceMixed = 1.2e-5, kReduceFp64 = 1e-5;
 extern "C" {
 static bool use_spatial(const sapb_dev *d, int ni, int nj);  // defined with the C ABI below
 }
@@ -412,6 +415,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call, bool lists) 
   const SliceCost cost = d->prec == DOUBLE ? kCostFp64
                          : spatial         ? (alone ? kAloneSpatial : kCostSpatial)
                                            : (alone ? kAloneAddress : kCostAddress);
+  const double reduce = call == Call::pinned ? 0.0 : d->prec == DOUBLE ? kReduceFp64 : kReduceMixed;
   const Shape sh = d->tpi ? Shape{d->tpi, d->ip}
                           : d->prec == DOUBLE ? shape_fp64(d->order, ni, nj) : shape_mixed(d, ni, nj, call, lists);
   const int tpi = sh.tpi, ip = sh.ip;
@@ -433,7 +437,7 @@ static Plan make_plan(const sapb_dev *d, int ni, int nj, Call call, bool lists) 
     const double used = std::min<double>(bps, ceil(B / sms)) / bps;
     double t = tiles * sqrt(used) * tile_time;
     if (ns > 1)
-      t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12) + (call == Call::pinned ? 0.0 : kReduceS);
+      t += ns * (kSliceS + (double)ni * kResStride * 8.0 / 4.0e12) + reduce;
     if (t < best_t * (best_t < 1e299 ? cost.more : 1.0)) {
       best_t = t;
       best = Plan{tpi, ip, ns, i_tiles, st};
